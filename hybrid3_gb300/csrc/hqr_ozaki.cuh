@@ -172,16 +172,37 @@ __device__ __forceinline__ uint32_t idesc_bf16(int M, int N) {
   return (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(N >> 3) << 17) |
          ((uint32_t)(M >> 4) << 24);
 }
+// MMAs and their commits are issued by one elected lane of a converged warp
+// (every lane executes the instruction, predicated): the operands then stay
+// in uniform registers.  Issued from a `lane == 0` branch each MMA cost 45
+// cycles in operand moves, whatever its size.
+// COLLECT: kAFill keeps the left operand in the tensor core's collector buffer,
+// kAUse and kALast take it from there instead of shared memory (M 128, N 64, K
+// 16: 35.6 cycles an MMA; 48.6, the shared-memory read of both operands,
+// without; 32 is the tensor work).
+enum ACollect : int { kARead = 0, kAFill = 1, kAUse = 2, kALast = 3 };
+template <int COLLECT>
 __device__ __forceinline__ void mma_bf16(uint32_t d_tmem, uint64_t a, uint64_t b, uint32_t id,
                                          uint32_t accumulate) {
-  asm volatile(
-      "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
-      "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}" ::"r"(d_tmem),
-      "l"(a), "l"(b), "r"(id), "r"(accumulate));
+#define HQR_MMA_BF16(USE)                                                                  \
+  asm volatile(                                                                            \
+      "{\n\t.reg .pred p, l;\n\telect.sync _|l, 0xffffffff;\n\tsetp.ne.b32 p, %4, 0;\n\t"   \
+      "@l tcgen05.mma.cta_group::1.kind::f16" USE " [%0], %1, %2, %3, p;\n\t}" ::"r"(d_tmem), \
+      "l"(a), "l"(b), "r"(id), "r"(accumulate))
+  if (COLLECT == kAFill)
+    HQR_MMA_BF16(".collector::a::fill");
+  else if (COLLECT == kAUse)
+    HQR_MMA_BF16(".collector::a::use");
+  else if (COLLECT == kALast)
+    HQR_MMA_BF16(".collector::a::lastuse");
+  else
+    HQR_MMA_BF16("");
+#undef HQR_MMA_BF16
 }
 __device__ __forceinline__ void mma_commit(uint64_t* bar) {
   asm volatile(
-      "tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(
+      "{\n\t.reg .pred l;\n\telect.sync _|l, 0xffffffff;\n\t"
+      "@l tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n\t}" ::"r"(
           smem_u32(bar))
       : "memory");
 }
@@ -296,7 +317,7 @@ struct Ctx {
   double* sY;           // the right operand: kK x kN doubles, ld kLdY
   uint32_t tmem;        // base of the 512 TMEM columns
   int n;                // K chunks consumed so far in this task (same in every thread)
-  int na;               // K chunks whose A copy has been issued (thread 0 only)
+  int na;               // K chunks whose A copy has been issued (warp 0 only)
   int yb;               // which half of sEb describes sY
   unsigned* err;        // scheduler error word
 };
@@ -472,19 +493,20 @@ __device__ __forceinline__ bool wait_chunk(const Ctx& c, int base, int stages, i
   return mbar_wait(c.bar + base + n % stages, (uint32_t)((n / stages) & 1), c.err);
 }
 // Chunk `chunk` of X into A stage n: its digit planes 0..G-1 (the first G x 4
-// KiB of the chunk).
+// KiB of the chunk).  Warp 0, one lane of which issues the copy.
 template <int G = kGroups>
 __device__ __forceinline__ void issue_a(Ctx& c, const uint8_t* X, int chunk, int n) {
+  if (threadIdx.x != 0) return;
   uint64_t* b = c.bar + kBarAFull + n % kAStages;
   mbar_expect_tx(b, G * kSliceABytes);
   tma_load_1d(c.sA + (n % kAStages) * kAChunkBytes, X + (size_t)chunk * kAChunkBytes, G * kSliceABytes, b);
 }
 
 // Issue the bulk copies of the first chunks of the next product's left
-// operand X (thread 0), e.g. before the right operand is staged.
+// operand X (warp 0), e.g. before the right operand is staged.
 template <int G = kGroups>
 __device__ __forceinline__ void prefetch(Ctx& c, const uint8_t* X) {
-  if (threadIdx.x == 0) {
+  if (threadIdx.x < 32) {
     fence_proxy_async_global();
     for (; c.na < c.n + kAStages; c.na++) issue_a<G>(c, X, c.na - c.n, c.na);
   }
@@ -497,8 +519,8 @@ __device__ __forceinline__ void slicer_sync() {
 
 // The 8 t-group accumulators of X (prepared slices) times the staged right
 // operand; Xnext (or nullptr): the left operand of the next product, whose
-// first chunks are fetched as soon as their stages are free.  Warp 0, one
-// thread: bulk copies of A and the MMAs; warps 1..7: slicing of B, up to
+// first chunks are fetched as soon as their stages are free.  Warp 0 (one
+// elected lane): bulk copies of A and the MMAs; warps 1..7: slicing of B, up to
 // kBStages chunks ahead of the MMAs.  On return (true) the accumulators are
 // final in TMEM.  G < 8: only the pairs of weight p + q < G (accumulators
 // 0..G-1; the others are left as they are).  nch: K chunks (8, or 16 for a
@@ -513,56 +535,58 @@ inline __device__ bool gemm(Ctx& c, const uint8_t* X, const uint8_t* Xnext, int 
   bool ok = true;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   if (warp == 0) {
-    if (lane == 0) {
-      const uint32_t id = idesc_bf16(kM, kN);
-      const uint64_t dA0 = sdesc(smem_u32(c.sA), 128, 256);
-      const uint64_t dB0 = sdesc(smem_u32(c.sB), 128, 256);
-      fence_proxy_async_global();
-      // chunks of this product not prefetched yet (stages free: every earlier MMA is done)
-      for (; c.na < n0 + kAStages; c.na++) issue_a<G>(c, X, c.na - n0, c.na);
-      for (int j = 0; j < nch && ok; j++) {
-        const int n = n0 + j;
-        if (!wait_chunk(c, kBarAFull, kAStages, n) || !wait_chunk(c, kBarBFull, kBStages, n)) {
-          ok = false;
-          break;
-        }
-        tc_fence_after();
-        const uint64_t dA = dA0 + (uint64_t)(((n % kAStages) * kAChunkBytes) >> 4);
-        const uint64_t dB = dB0 + (uint64_t)(((n % kBStages) * kBChunkBytes) >> 4);
-        // pairs (p, q) with p + q <= G - 1 into t-group p + q; the first
-        // product into each group in chunk 0 overwrites it
+    const uint32_t id = idesc_bf16(kM, kN);
+    const uint64_t dA0 = sdesc(smem_u32(c.sA), 128, 256);
+    const uint64_t dB0 = sdesc(smem_u32(c.sB), 128, 256);
+    fence_proxy_async_global();
+    // chunks of this product not prefetched yet (stages free: every earlier MMA is done)
+    for (; c.na < n0 + kAStages; c.na++) issue_a<G>(c, X, c.na - n0, c.na);
+    for (int j = 0; j < nch && ok; j++) {
+      const int n = n0 + j;
+      ok = wait_chunk(c, kBarAFull, kAStages, n) && wait_chunk(c, kBarBFull, kBStages, n);
+      ok = __all_sync(0xffffffffu, ok);
+      if (!ok) break;
+      tc_fence_after();
+      const uint64_t dA = dA0 + (uint64_t)(((n % kAStages) * kAChunkBytes) >> 4);
+      const uint64_t dB = dB0 + (uint64_t)(((n % kBStages) * kBChunkBytes) >> 4);
+      // pairs (p, q) with p + q <= G - 1 into t-group p + q; the first
+      // product into each group in chunk 0 overwrites it
 #pragma unroll
-        for (int p = 0; p < kS && p < G; p++) {
+      for (int p = 0; p < kS && p < G; p++) {
 #pragma unroll
-          for (int q = 0; q < kS && p + q < G; q++) {
-            const int first_p = (p + q) - (kS - 1) > 0 ? (p + q) - (kS - 1) : 0;
-            const uint32_t acc = (j > 0 || p > first_p) ? 1u : 0u;
-            mma_bf16(c.tmem + (uint32_t)((p + q) * kN), dA + (uint64_t)((p * kSliceABytes) >> 4),
-                     dB + (uint64_t)((q * kSliceBBytes) >> 4), id, acc);
-          }
-        }
-        mma_commit(c.bar + kBarDone + n % kDoneStages);
-        // refill the A stage of chunk n - 1 with chunk n - 1 + kAStages once its MMAs are done
-        if (j >= 1 && j + kAStages - 1 < nch) {
-          if (!wait_chunk(c, kBarDone, kDoneStages, n - 1)) {
-            ok = false;
-            break;
-          }
-          issue_a<G>(c, X, j + kAStages - 1, n + kAStages - 1);
-          c.na = n + kAStages;
+        for (int q = 0; q < kS && p + q < G; q++) {
+          const int first_p = (p + q) - (kS - 1) > 0 ? (p + q) - (kS - 1) : 0;
+          const uint32_t acc = (j > 0 || p > first_p) ? 1u : 0u;
+          const uint32_t d = c.tmem + (uint32_t)((p + q) * kN);
+          const uint64_t a = dA + (uint64_t)((p * kSliceABytes) >> 4), b = dB + (uint64_t)((q * kSliceBBytes) >> 4);
+          const int last_q = (G < kS ? G : kS) - 1 - p;   // slice p's last product
+          if (last_q == 0)
+            mma_bf16<kARead>(d, a, b, id, acc);
+          else if (q == 0)
+            mma_bf16<kAFill>(d, a, b, id, acc);
+          else if (q < last_q)
+            mma_bf16<kAUse>(d, a, b, id, acc);
+          else
+            mma_bf16<kALast>(d, a, b, id, acc);
         }
       }
-      // prefetch the next product's first chunks into the stages of the last kAStages
-      if (ok && Xnext) {
-        for (int j = 0; j < kAStages; j++) {
-          if (!wait_chunk(c, kBarDone, kDoneStages, n0 + nch - kAStages + j)) {
-            ok = false;
-            break;
-          }
-          issue_a<G>(c, Xnext, j, n0 + nch + j);
-        }
-        if (ok) c.na = n0 + nch + kAStages;
+      mma_commit(c.bar + kBarDone + n % kDoneStages);
+      // refill the A stage of chunk n - 1 with chunk n - 1 + kAStages once its MMAs are done
+      if (j >= 1 && j + kAStages - 1 < nch) {
+        ok = __all_sync(0xffffffffu, wait_chunk(c, kBarDone, kDoneStages, n - 1));
+        if (!ok) break;
+        issue_a<G>(c, X, j + kAStages - 1, n + kAStages - 1);
+        c.na = n + kAStages;
       }
+    }
+    // prefetch the next product's first chunks into the stages of the last kAStages
+    if (ok && Xnext) {
+      for (int j = 0; j < kAStages; j++) {
+        ok = __all_sync(0xffffffffu, wait_chunk(c, kBarDone, kDoneStages, n0 + nch - kAStages + j));
+        if (!ok) break;
+        issue_a<G>(c, Xnext, j, n0 + nch + j);
+      }
+      if (ok) c.na = n0 + nch + kAStages;
     }
     __syncwarp();
   } else {
