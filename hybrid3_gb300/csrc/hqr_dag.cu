@@ -173,17 +173,22 @@ static int run_dag(DagParams& p, DagWorkspace* ws, const Geometry& g, cudaStream
 // run in phases (DagParams::ts_split).
 constexpr long long kPhasedWork = 6000;
 
-// 64-column chunks per split update task, run one after the other: two (a
+// 64-column chunks per split update task, run one after the other.  Two (a
 // whole 128-column tile) halve the number of update tasks and with them the
-// scheduling round trips (a queue claim and the dependents' releases, about
-// 6 us per task), at the price of half the tasks per step.
-constexpr int kOzChunksPerTask = 2;
-static void set_oz(DagParams& p, const Geometry& g, const OzWorkspace* oz) {
+// scheduling round trips (a queue claim and the dependents' releases, about 6
+// us per task).  One, where the longest chain of whole-tile updates (`path`
+// tasks) takes longer than all `tiles` of them on every SM: the chain's time
+// halves (Q^T C and Q C, n = 8192, 512 columns: 21.5 -> 13.3 ms together).  C with data in one
+// chunk only (ccols) has nothing to cut.
+static int oz_chunks(long long tiles, long long path, long long ccols = 0) {
+  return (ccols > 0 && ccols <= oz::kN) || tiles >= path * dag_sm_count() ? 2 : 1;
+}
+static void set_oz(DagParams& p, const Geometry& g, const OzWorkspace* oz, int chunks) {
   if (oz && oz->slices) {
     p.oz = 1;
     p.oz_groups = oz->groups;
     p.oz_p32 = oz->fp32_panels;
-    p.oz_cpt = kOzChunksPerTask;
+    p.oz_cpt = chunks;
     p.NC = g.NB / oz::kN / p.oz_cpt;
     p.slices = oz->slices;
     p.sexp = oz->sexp;
@@ -224,7 +229,10 @@ int launch_factor(const Geometry& g, DagWorkspace* ws, double* dA, double* dT, d
   p.TAU = dTAU;
   p.C = dA;
   p.timeout_ns = timeout_ns;
-  set_oz(p, g, ozw);
+  long long tiles = 0;
+  for (int i = 0; i < g.steps; i++) tiles += (long long)(g.NT - 1 - i) * (g.MT - i);
+  const int chain = tw && tw->S > 0 && tw->S < g.MT ? tw->S + (g.MT + tw->S - 1) / tw->S : g.MT;   // tasks down a column
+  set_oz(p, g, ozw, oz_chunks(tiles, chain + g.steps));
   p.prep = p.oz;
   p.nblk = g.NB / g.w;
   set_tree(p, g, tw);
@@ -271,7 +279,9 @@ int launch_apply_qt(const Geometry& g, DagWorkspace* ws, const double* dA, doubl
   p.TAU = const_cast<double*>(dTAU);
   p.C = dC;
   p.timeout_ns = timeout_ns;
-  set_oz(p, g, ozw);
+  long long tiles = 0;
+  for (int i = 0; i < g.steps; i++) tiles += (long long)CT * (g.MT - i);
+  set_oz(p, g, ozw, oz_chunks(tiles, g.MT + g.steps, ccols));
   p.prep = 0;
   p.nblk = 1;
   // rebuild_t: panel tasks rebuild each panel tile's T (FP64: its diagonal
@@ -300,7 +310,9 @@ int launch_apply_qt_tree(const Geometry& g, DagWorkspace* ws, const double* dA, 
   p.TAU = const_cast<double*>(dTAU);
   p.C = dC;
   p.timeout_ns = timeout_ns;
-  set_oz(p, g, ozw);
+  long long tiles = 0;
+  for (int i = 0; i < g.steps; i++) tiles += (long long)CT * (g.MT - i);
+  set_oz(p, g, ozw, oz_chunks(tiles, tw->S + (g.MT + tw->S - 1) / tw->S + g.steps));
   p.prep = 0;
   p.nblk = 1;
   p.skip_panels = 1;   // the T factors / slices of the factorization on this plan
@@ -326,7 +338,9 @@ int launch_build_q(const Geometry& g, DagWorkspace* ws, const double* dA, double
   p.TAU = const_cast<double*>(dTAU);
   p.C = dQ;
   p.timeout_ns = timeout_ns;
-  set_oz(p, g, ozw);
+  long long tiles = 0;
+  for (int i = 0; i < g.steps; i++) tiles += (long long)(g.NT - i) * (g.MT - i);
+  set_oz(p, g, ozw, oz_chunks(tiles, g.MT + g.steps));
   p.prep = 0;
   p.nblk = 1;
   p.skip_panels = rebuild_t ? 0 : 1;   // as in launch_apply_qt (split: T from its own slot)
@@ -355,7 +369,9 @@ int launch_apply_q(const Geometry& g, DagWorkspace* ws, const double* dA, double
   p.TAU = const_cast<double*>(dTAU);
   p.C = dC;
   p.timeout_ns = timeout_ns;
-  set_oz(p, g, ozw);
+  long long tiles = 0;
+  for (int i = 0; i < g.steps; i++) tiles += (long long)CT * (g.MT - i);
+  set_oz(p, g, ozw, oz_chunks(tiles, g.MT + g.steps, ccols));
   p.prep = 0;
   p.nblk = 1;
   p.skip_panels = rebuild_t ? 0 : 1;
