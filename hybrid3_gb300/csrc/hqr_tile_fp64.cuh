@@ -90,20 +90,6 @@ template <> struct PanelReal<float> {
   static constexpr float kSsLo = 1e-34f, kSsHi = 1e34f;
 };
 
-template <typename R>
-__device__ __forceinline__ R block_max(R v, R* red) {
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) v = fmax(v, __shfl_xor_sync(0xffffffffu, v, o));
-  const int w = threadIdx.x >> 5, l = threadIdx.x & 31;
-  __syncthreads();
-  if (l == 0) red[w] = v;
-  __syncthreads();
-  R s = R(0);
-#pragma unroll
-  for (int i = 0; i < kWarps; i++) s = fmax(s, red[i]);
-  return s;
-}
-
 // The scalar part of dlarfg for alpha = a, ||x|| = xnorm, ss = ||x||^2; plain:
 // ss lies where its square root needs no scaling.  beta = -sign(a) ||[a; x]||,
 // tau = (beta - a) / beta, scal = 1 / (a - beta) (x is scaled by scal after
@@ -140,62 +126,8 @@ __device__ __forceinline__ void larfg_scalars(R a, R xnorm, R ss, bool plain, R&
   }
 }
 
-__device__ void block_larfg(double* alpha, double* x, int n, double* tau_out, double* red) {
-  double ss = 0.0;
-  for (int r = threadIdx.x; r < n; r += kThreads) {
-    const double v = x[r];
-    ss = fma(v, v, ss);
-  }
-  ss = block_sum(ss, red);
-  double xnorm;
-  bool plain = false;   // ||x||^2 and alpha^2 in range: beta from the squared norms directly
-  if (ss == 0.0) {
-    xnorm = 0.0;
-  } else if (ss >= 1e-290 && ss <= 1e290) {
-    xnorm = sqrt(ss);
-    plain = true;
-  } else {  // scaled norm, as LAPACK dnrm2 does, for tiny or huge columns
-    double amax = 0.0;
-    for (int r = threadIdx.x; r < n; r += kThreads) amax = fmax(amax, fabs(x[r]));
-    amax = block_max(amax, red);
-    double s2 = 0.0;
-    for (int r = threadIdx.x; r < n; r += kThreads) {
-      const double v = x[r] / amax;
-      s2 = fma(v, v, s2);
-    }
-    s2 = block_sum(s2, red);
-    xnorm = amax * sqrt(s2);
-  }
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    double tau, scal, beta;
-    int knt;
-    larfg_scalars(*alpha, xnorm, ss, plain, tau, scal, knt, beta);
-    red[kBcast + 0] = tau;
-    red[kBcast + 1] = scal;
-    red[kBcast + 2] = (double)knt;
-    red[kBcast + 3] = beta;
-  }
-  __syncthreads();
-  const double tau = red[kBcast + 0], scal = red[kBcast + 1];
-  const int knt = (int)red[kBcast + 2];
-  if (tau != 0.0) {
-    const double rsafmn = 1.0 / (DBL_MIN / (DBL_EPSILON * 0.5));
-    for (int r = threadIdx.x; r < n; r += kThreads) {
-      double v = x[r];
-      for (int j = 0; j < knt; j++) v *= rsafmn;
-      x[r] = v * scal;
-    }
-  }
-  if (threadIdx.x == 0) {
-    *alpha = red[kBcast + 3];
-    *tau_out = tau;
-  }
-  __syncthreads();
-}
-
-// dlarfg on [alpha; x] by one warp (x: n contiguous shared doubles), with the
-// arithmetic of block_larfg; every lane computes the (identical) scalars.
+// dlarfg on [alpha; x] by one warp (x: n contiguous shared doubles); every
+// lane computes the (identical) scalars.
 template <typename R>
 __device__ void warp_larfg(R* alpha, R* x, int n, R* tau_out) {
   using K = PanelReal<R>;
@@ -368,7 +300,7 @@ __device__ void t_from_gram(const RT* G, const RT* tau, RT* T, int w) {
 // memory.  unit: V is unit lower (rows 0..w-1 hold the unit triangle, V(c,c)
 // = 1 implicit); otherwise V is dense (TS block, top part = identity).
 // G (w x w scratch) receives the needed Gram entries.  T (w x w, ld w) output.
-__device__ void build_t_block(const double* V, int ldv, int m, int w, bool unit, const double* tau,
+inline __device__ void build_t_block(const double* V, int ldv, int m, int w, bool unit, const double* tau,
                               double* G, double* T) {
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int npairs = w * (w - 1) / 2;
@@ -542,13 +474,35 @@ constexpr unsigned kPanelMaxHi = kHiExp(450);
 // columns; warp 4 forms T's column c during step c + 1 (T(0:c, c) = -tau_c
 // T(0:c, 0:c) G(0:c, c)).  A column whose norm or alpha is outside the plain
 // range (spec) is scaled to v by warp 0 and its dots are taken again.
-template <bool TS>
-__device__ __forceinline__ void panel_qr(double* R, int ldr, double* A, int lda, int m, int w, double* tau,
-                                         double* scal, int* spec, double* G, double* T) {
+//
+// Larfg: the reflector's convention (LapackLarfg, or tile_kernel.h's).  nref:
+// reflectors formed (columns from there on are updated only).  GRAM false: no
+// Gram entries and no T.
+struct LapackLarfg {
+  // false: outside the plain range (2^-960 <= ss < 2^960, alpha zero or 2^-465
+  // .. 2^465), read off the high words: an FP64 comparison is an FP64
+  // instruction too
+  __device__ static bool scalars(double a, double ss, double& tau, double& scal, double& beta) {
+    const unsigned sh = (unsigned)__double2hiint(ss), ah = (unsigned)__double2hiint(a) & 0x7fffffffu;
+    tau = 0.0;
+    scal = 1.0;
+    beta = a;
+    if (sh >= kHiExp(-960) && sh < kHiExp(960) && ah < kHiExp(465) &&
+        (ah >= kHiExp(-465) || (ah | (unsigned)__double2loint(a)) == 0u)) {
+      larfg_newton(a, ss, tau, scal, beta);
+      return true;
+    }
+    return (sh | (unsigned)__double2loint(ss)) == 0u;   // x = 0: H = I
+  }
+};
+template <bool TS, class Larfg = LapackLarfg, bool GRAM = true>
+__device__ __forceinline__ void panel_qr(double* R, int ldr, double* A, int lda, int m, int w, int nref,
+                                         double* tau, double* scal, int* spec, double* G, double* T) {
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  constexpr int kParty = (kPanelWorkers + 1) * 32;
+  constexpr int kParty = (kPanelWorkers + 1) * 32;                 // the workers and warp 0
+  constexpr int kStepParty = (kPanelWorkers + (GRAM ? 1 : 0)) * 32;   // the workers (and warp 4)
   if (warp == 0) {
-    for (int c = 0; c < w; c++) {
+    for (int c = 0; c < nref; c++) {
       if (c > 0) bar_sync<kBarColumn, 64>();
       double* x = A + (size_t)c * lda;
       double* al = TS ? R + c + (size_t)c * ldr : x + c;
@@ -568,14 +522,8 @@ __device__ __forceinline__ void panel_qr(double* R, int ldr, double* A, int lda,
       }
       warp_sums_fixed(ssv);
       const double ss = ssv[0];
-      // the plain range (2^-960 <= ss < 2^960, alpha zero or 2^-465 .. 2^465),
-      // from the high words: an FP64 comparison is an FP64 instruction too
-      const unsigned sh = (unsigned)__double2hiint(ss), ah = (unsigned)__double2hiint(a) & 0x7fffffffu;
-      const bool plain = sh >= kHiExp(-960) && sh < kHiExp(960) && ah < kHiExp(465) &&
-                         (ah >= kHiExp(-465) || (ah | (unsigned)__double2loint(a)) == 0u);
-      double t = 0.0, sc = 1.0, beta = a;
-      if (plain) larfg_newton(a, ss, t, sc, beta);
-      const bool special = !plain && (sh | (unsigned)__double2loint(ss)) != 0u;
+      double t, sc, beta;
+      const bool special = !Larfg::scalars(a, ss, t, sc, beta);
       __syncwarp();
       if (!special) {
         if (lane == 0) {
@@ -596,8 +544,8 @@ __device__ __forceinline__ void panel_qr(double* R, int ldr, double* A, int lda,
       }
     }
   } else if (warp == 4) {
-    for (int c = 0; c < w; c++) {
-      bar_sync<kBarStep, kParty>();
+    for (int c = 0; GRAM && c < nref; c++) {
+      bar_sync<kBarStep, kStepParty>();
       double s = 0.0;
       if (lane < c)
         for (int b = 0; b < c; b++) s = fma(lane <= b ? T[lane + b * w] : 0.0, G[b + c * w], s);
@@ -608,9 +556,9 @@ __device__ __forceinline__ void panel_qr(double* R, int ldr, double* A, int lda,
     }
   } else {
     const int wi = warp < 4 ? warp - 1 : warp - 2;
-    for (int c = 0; c < w; c++) {
+    for (int c = 0; c < nref; c++) {
       // items 0 .. w - 2 - c: columns c + 1 .. w - 1; then columns 0 .. c - 1
-      const int nupd = w - 1 - c;
+      const int nupd = w - 1 - c, items = GRAM ? w - 1 : nupd;
       const int r0 = TS ? 0 : c + 1;
       const double* x = A + (size_t)c * lda;
       double acc[kPanelGroups][kPanelItems];
@@ -619,12 +567,12 @@ __device__ __forceinline__ void panel_qr(double* R, int ldr, double* A, int lda,
       auto dots = [&]() {
 #pragma unroll
         for (int g = 0; g < kPanelGroups; g++) {
-          if (item(g, 0) >= w - 1) break;
+          if (item(g, 0) >= items) break;
           const double* aq[kPanelItems];   // (past the last item: column c, the result unused)
 #pragma unroll
           for (int q = 0; q < kPanelItems; q++) {
             acc[g][q] = 0.0;
-            aq[q] = A + (size_t)(item(g, q) < w - 1 ? column(item(g, q)) : c) * lda;
+            aq[q] = A + (size_t)(item(g, q) < items ? column(item(g, q)) : c) * lda;
           }
           for (int rb = r0 & ~127; rb < m; rb += 32 * kPanelRows) {
             double xv[kPanelRows], av[kPanelItems][kPanelRows];
@@ -641,7 +589,7 @@ __device__ __forceinline__ void panel_qr(double* R, int ldr, double* A, int lda,
               if (rb + 32 * i < m && rb + 32 * i + 31 >= r0)
 #pragma unroll
                 for (int q = 0; q < kPanelItems; q++)
-                  if (q < kPanelItems - 1 || item(g, q) < w - 1) acc[g][q] = fma(xv[i], av[q][i], acc[g][q]);
+                  if (q < kPanelItems - 1 || item(g, q) < items) acc[g][q] = fma(xv[i], av[q][i], acc[g][q]);
           }
           warp_sums_fixed(acc[g]);
         }
@@ -652,8 +600,8 @@ __device__ __forceinline__ void panel_qr(double* R, int ldr, double* A, int lda,
       for (int g = 0; g < kPanelGroups; g++) {
         const int it = item(g, lane < kPanelItems ? lane : 0);
         rc[g] = mul[g] = 0.0;
-        if (it < w - 1 && (it < nupd || !TS)) rc[g] = R[c + (size_t)column(it) * ldr];
-        if (it < w - 1 && it >= nupd) mul[g] = scal[it - nupd];
+        if (it < items && (it < nupd || !TS)) rc[g] = R[c + (size_t)column(it) * ldr];
+        if (it < items && it >= nupd) mul[g] = scal[it - nupd];
       }
       dots();
       bar_sync<kBarScalars, kParty>();
@@ -665,7 +613,7 @@ __device__ __forceinline__ void panel_qr(double* R, int ldr, double* A, int lda,
       const bool moves = __double_as_longlong(t) != 0;
 #pragma unroll
       for (int g = 0; g < kPanelGroups; g++) {
-        if (item(g, 0) >= w - 1) break;
+        if (item(g, 0) >= items) break;
         const int mine = item(g, lane < kPanelItems ? lane : 0);
         double d = acc[g][0];
 #pragma unroll
@@ -673,7 +621,7 @@ __device__ __forceinline__ void panel_qr(double* R, int ldr, double* A, int lda,
         // update: s = tau (v_c . a_j + r_cj); Gram: G(b, c) = v_b . v_c
         const double s = fma(sc, d, rc[g]) * (mine < nupd ? t : mul[g]);
         const double f = s * sc;
-        if (lane < kPanelItems && mine < w - 1) {
+        if (lane < kPanelItems && mine < items) {
           if (mine < nupd)
             R[c + (size_t)(c + 1 + mine) * ldr] = rc[g] - s;
           else
@@ -703,13 +651,13 @@ __device__ __forceinline__ void panel_qr(double* R, int ldr, double* A, int lda,
               }
             }
           }
-          if (it == 0) {
+          if (it == 0 && c + 1 < nref) {
             __syncwarp();
             bar_arrive<kBarColumn, 64>();
           }
         }
       }
-      bar_sync<kBarStep, kParty>();
+      bar_sync<kBarStep, kStepParty>();
     }
   }
   __syncthreads();
@@ -959,7 +907,7 @@ __device__ void task_geqrt_blk(double* A, double* T, double* tau_g, const TileSh
       note_top(load_panel(sP, NB, A + i0 + (size_t)i0 * NB, NB, m, w), s_top);
       __syncthreads();
       if (*s_top < kPanelMaxHi)
-        panel_qr<false>(sP, NB, sP, NB, m, w, sTau, scal, spec, sG, sTb);
+        panel_qr<false>(sP, NB, sP, NB, m, w, w, sTau, scal, spec, sG, sTb);
       else
         panel_qr_general<false>(sP, NB, sP, NB, m, w, sTau, scal, sG, sTb);
       // R and V = x scal to the tile; V also to the trailing update's buffers
@@ -1008,12 +956,6 @@ __device__ void task_geqrt_blk(double* A, double* T, double* tau_g, const TileSh
   __syncthreads();
 }
 
-// CORE_dgeqrt(NB, NB, IB, A, NB, T, NB, TAU)
-__device__ void task_geqrt(double* A, double* T, double* tau_g, const TileShape& sh, double* smem,
-                           const SmemPlan& sp) {
-  for (int b = 0; b < sh.NB / sh.w; b++) task_geqrt_blk(A, T, tau_g, sh, smem, sp, b);
-}
-
 // Inner block b of CORE_dtsqrt(NB, NB, IB, A1, NB, A2, NB, T, NB, TAU): A1
 // holds R (upper part) above the GEQRT's V (strict lower part, left
 // untouched).  The QR of [R(bw:(b+1)w, bw:(b+1)w); A2(:, bw:(b+1)w)] (blocks
@@ -1052,7 +994,7 @@ __device__ void task_tsqrt_blk(double* A1, double* A2, double* T, double* tau_g,
       note_top(max(top, load_panel(sR, w, A1 + i0 + (size_t)i0 * NB, NB, w, w, 0)), s_top);
       __syncthreads();
       if (*s_top < kPanelMaxHi)
-        panel_qr<true>(sR, w, sA, NB, NB, w, sTau, scal, spec, sG, sTb);
+        panel_qr<true>(sR, w, sA, NB, NB, w, w, sTau, scal, spec, sG, sTb);
       else
         panel_qr_general<true>(sR, w, sA, NB, NB, w, sTau, scal, sG, sTb);
       // V = x scal to the tile (a merge: its upper triangle) and to the
@@ -1115,16 +1057,10 @@ __device__ void task_tsqrt_blk(double* A1, double* A2, double* T, double* tau_g,
   __syncthreads();
 }
 
-// CORE_dtsqrt(NB, NB, IB, A1, NB, A2, NB, T, NB, TAU)
-__device__ void task_tsqrt(double* A1, double* A2, double* T, double* tau_g, const TileShape& sh,
-                           double* smem, const SmemPlan& sp) {
-  for (int b = 0; b < sh.NB / sh.w; b++) task_tsqrt_blk(A1, A2, T, tau_g, sh, smem, sp, b);
-}
-
 // CORE_dormqr(Left, Trans, NB, ncol, NB, IB, V, NB, T, NB, C, NB) on columns
 // [c0, c0+ncol) of C (notrans: CORE_dormqr(Left, NoTrans, ...), the inner
 // blocks in reverse order).
-__device__ void task_larfb(const double* V, const double* T, double* C, int c0, int ncol,
+inline __device__ void task_larfb(const double* V, const double* T, double* C, int c0, int ncol,
                            const TileShape& sh, double* smem, const SmemPlan& sp, bool notrans = false) {
   const int NB = sh.NB, w = sh.w;
   double* sC = smem + sp.off_c1;
@@ -1144,7 +1080,7 @@ __device__ void task_larfb(const double* V, const double* T, double* C, int c0, 
 // T, NB) on columns [c0, c0+ncol) of A1 and A2 (notrans: Left, NoTrans, the
 // inner blocks in reverse order).  v_upper: CORE_dttmqr, V is the upper
 // triangle (with the diagonal) of its tile.
-__device__ void task_ssrfb(double* A1, double* A2, const double* V, const double* T, int c0,
+inline __device__ void task_ssrfb(double* A1, double* A2, const double* V, const double* T, int c0,
                            int ncol, const TileShape& sh, double* smem, const SmemPlan& sp,
                            bool notrans = false, bool v_upper = false) {
   const int NB = sh.NB, w = sh.w;

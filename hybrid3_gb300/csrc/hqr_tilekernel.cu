@@ -1,8 +1,13 @@
 // hqr_tilekernel.cu -- the reference's per-tile kernels (tile_kernel.h:28-230,
 // bodies tile_kernel.c:19-716) with their own conventions, on the GPU.
 //
-// Each entry point runs one CTA of kThreads FP64 threads on one tile (or tile
-// pair) in device memory.  Host pointers are staged through a device scratch
+// The column loops (dgeqr2, dtsqr2) run on one CTA with the panel in shared
+// memory (the factorization's loop, hqr_tile_fp64.cuh, with this file's
+// reflector convention); the T factors and the applications, whose columns are
+// independent, spread them over the SMs.  One panel step of a tile driver
+// (dgeqrt, dlarft, dlarfb, dtsqrt, dlarft, dssrfb) at order 128, block 32:
+// 1.40 ms; 12.4 ms with every kernel on one CTA and its operands in global
+// memory.  Host pointers are staged through a device scratch
 // pool for the call (copied in, and back out for every array the function may
 // write); device and managed pointers are used in place.  The calls are
 // synchronous, like the reference's.  Conventions (which differ from the
@@ -23,14 +28,75 @@
 
 #include "hqr_common.cuh"
 #include "hqr_internal.h"
+#include "hqr_tile_fp64.cuh"
 #include "tile_kernel.h"
 
 namespace hqr {
 namespace tk {
 
 // ---------------------------------------------------------------------------
-// Device kernels (one CTA each)
+// Device kernels
 // ---------------------------------------------------------------------------
+
+// The reflector of this file's kernels: beta = +sqrt(a^2 + ss), head = a -
+// beta, v = x / head, tau = 2 head^2 / (head^2 + ss); no guard (x = 0 and a > 0
+// divides by zero, as the reference does).
+struct TileLarfg {
+  __device__ static bool scalars(double a, double ss, double& tau, double& scal, double& beta) {
+    beta = sqrt(ss + a * a);
+    const double head = a - beta;
+    scal = 1.0 / head;
+    tau = 2.0 / (head * head + ss) * head * head;
+    return true;
+  }
+};
+
+// Doubles of shared memory of k_panel beyond its row x col panel.
+constexpr int kPanelExtra = 2 * kMaxW + kMaxW / 2 + kMaxW * kMaxW;
+constexpr size_t kPanelSmem = 220 * 1024;
+// The widest panel (at most kMaxW columns) of `row` rows that fits (0: none).
+int panel_cols(int row) {
+  const long fit = ((long)kPanelSmem / 8 - kPanelExtra) / (row > 0 ? row : 1);
+  return (int)(fit > kMaxW ? kMaxW : fit);
+}
+
+// The column loop on a panel of at most kMaxW columns, one CTA.  TS:
+// tile_sub_dtsqr2 on [A1 (upper col x col); A2], A2 becomes V.  !TS:
+// tile_sub_dgeqr2 on A2 (row x col) alone, V also to Y (ld lda, unit
+// diagonal); a square panel has no last reflector (TAU(col-1) is left as it
+// is and Y(col-1, col-1) = 0).  The loop's FP64 work (4 row col^2 flops on one
+// SM) and its chain of col norms bound it.
+template <bool TS>
+__global__ void __launch_bounds__(kThreads) k_panel(int row, int col, double* A1, int lda1, double* A2, int lda2,
+                                                    double* TAU, double* Y) {
+  extern __shared__ double sm[];
+  double* sA = sm;
+  double* tau = sA + (size_t)row * col;
+  double* scal = tau + kMaxW;
+  int* spec = reinterpret_cast<int*>(scal + kMaxW);
+  double* sR = scal + kMaxW + kMaxW / 2;
+  for (int e = threadIdx.x; e < row * col; e += kThreads) sA[e] = A2[e % row + (size_t)(e / row) * lda2];
+  if (TS)
+    for (int e = threadIdx.x; e < col * col; e += kThreads)
+      sR[e] = (e % col <= e / col) ? A1[e % col + (size_t)(e / col) * lda1] : 0.0;
+  __syncthreads();
+  const int nref = (!TS && row == col) ? col - 1 : col;
+  if (TS)
+    panel_qr<true, TileLarfg, false>(sR, col, sA, row, row, col, nref, tau, scal, spec, nullptr, nullptr);
+  else
+    panel_qr<false, TileLarfg, false>(sA, row, sA, row, row, col, nref, tau, scal, spec, nullptr, nullptr);
+  for (int e = threadIdx.x; e < row * col; e += kThreads) {
+    const int r = e % row, c = e / row;
+    double v = sA[e];
+    if (c < nref && (TS || r > c)) v *= scal[c];
+    A2[r + (size_t)c * lda2] = v;
+    if (!TS && r >= c) Y[r + (size_t)c * lda2] = c >= nref ? 0.0 : (r == c ? 1.0 : v);
+  }
+  if (TS)
+    for (int e = threadIdx.x; e < col * col; e += kThreads)
+      if (e % col <= e / col) A1[e % col + (size_t)(e / col) * lda1] = sR[e];
+  for (int c = threadIdx.x; c < nref; c += kThreads) TAU[c] = tau[c];
+}
 
 // out[c] = sum_{r < n} x[r] * (base + c*ld)[r] for c < nc: one warp per column.
 __device__ void col_dots(const double* x, const double* base, int ld, int n, int nc, double* out) {
@@ -187,49 +253,69 @@ __global__ void __launch_bounds__(kThreads) k_sub_dtsqr2(int row, int col, doubl
   if (tid == 0) TAU[i] = t * y_head * y_head;
 }
 
-// tile_sub_dlarft (tile_kernel.c:220-262): lower T (ld ldt) from Y (ld lda,
-// all `row` rows as stored) and TAU.  G: col x col global scratch.
-__global__ void __launch_bounds__(kThreads) k_sub_dlarft(int row, int col, const double* Y, int lda,
-                                                          const double* TAU, double* T, int ldt, double* G,
-                                                          int transpose_out) {
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  // G(i, c) = Y(:,i)^T Y(:,c) for c < i
-  const int npairs = col * (col - 1) / 2;
-  for (int p = warp; p < npairs; p += kWarps) {
-    int i = 1, base = 0;
-    while (base + i <= p) {
-      base += i;
-      i++;
+// G(i, c) = Y(:, i)^T Y(:, c), c < i, to G[i col + c]: block i, four columns c
+// of a warp at a time.  lower: Y is unit lower (what is stored above its
+// diagonal is not read).
+__global__ void __launch_bounds__(kThreads) k_gram(int row, int col, const double* __restrict__ Y, int lda,
+                                                   double* __restrict__ G, int lower) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int i = blockIdx.x;
+  const double* yi = Y + (size_t)i * lda;
+  for (int c0 = 4 * warp; c0 < i; c0 += 4 * kWarps) {
+    double s[4] = {0.0, 0.0, 0.0, 0.0};
+    for (int r = (lower ? i : 0) + lane; r < row; r += 32) {
+      const double x = yi[r];
+#pragma unroll
+      for (int q = 0; q < 4; q++)
+        if (c0 + q < i) s[q] = fma(x, Y[r + (size_t)(c0 + q) * lda], s[q]);
     }
-    const int c = p - base;
-    const double* yi = Y + (size_t)i * lda;
-    const double* yc = Y + (size_t)c * lda;
-    double s = 0.0;
-    for (int r = lane; r < row; r += 32) s = fma(yi[r], yc[r], s);
-    s = warp_sum(s);
-    if (lane == 0) G[i + (size_t)c * col] = s;
+    warp_sums_fixed(s);
+#pragma unroll
+    for (int q = 0; q < 4; q++)
+      if (c0 + q < i && lane == q) G[(size_t)i * col + c0 + q] = s[q];
   }
-  for (int i = tid; i < col; i += kThreads) T[i + (size_t)i * ldt] = TAU[i];
-  __syncthreads();
-  for (int i = 1; i < col; i++) {
-    const double alpha = -T[i + (size_t)i * ldt];
-    for (int r = tid; r < i; r += kThreads) {
-      double s = 0.0;
-      for (int c = 0; c < i; c++) s = fma(T[c + (size_t)r * ldt], G[i + (size_t)c * col], s);
-      T[i + (size_t)r * ldt] = alpha * s;
+}
+
+// tile_sub_dlarft (tile_kernel.c:220-262): lower T (ld ldt) from G and TAU:
+// T(i, r) = -tau_i sum_{c < i} T(c, r) G(i, c) for r < i.  Column r depends on
+// its own elements only: one warp per column, its elements t in shared memory
+// (col doubles a warp), four rows i at a time: the dots with the t known
+// before them together, then the four in turn.  zero_upper: T's strict upper
+// part counts as zero instead of as stored; transposed: T(i, r) is stored at
+// (r, i).
+__global__ void __launch_bounds__(kThreads) k_larft_cols(int col, const double* __restrict__ G,
+                                                         const double* __restrict__ TAU, double* T, int ldt,
+                                                         int zero_upper, int transposed) {
+  extern __shared__ double sm[];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int r = blockIdx.x * (blockDim.x >> 5) + warp;
+  if (r >= col) return;
+  double* t = sm + (size_t)warp * col;
+  for (int c = lane; c < col; c += 32)
+    t[c] = c == r ? TAU[r] : (c < r && !zero_upper ? T[c + (size_t)r * ldt] : 0.0);
+  __syncwarp();
+  for (int i0 = (r + 1) & ~3; i0 < col; i0 += 4) {
+    double s[4] = {0.0, 0.0, 0.0, 0.0};
+    for (int c = lane; c < i0; c += 32) {
+      const double tc = t[c];
+#pragma unroll
+      for (int q = 0; q < 4; q++)
+        if (i0 + q < col) s[q] = fma(tc, G[(size_t)(i0 + q) * col + c], s[q]);
     }
-    __syncthreads();
-  }
-  if (transpose_out) {
-    // T holds the lower T here (a zeroed scratch); move it to the upper part
-    for (int e = tid; e < col * col; e += kThreads) {
-      const int r = e % col, c = e / col;
-      if (r > c) {
-        T[c + (size_t)r * ldt] = T[r + (size_t)c * ldt];
-        T[r + (size_t)c * ldt] = 0.0;
-      }
+    warp_sums_fixed(s);
+    double v[4];   // t(i0 + q)
+#pragma unroll
+    for (int q = 0; q < 4; q++) {
+      const int i = i0 + q;
+      if (i >= col) break;
+#pragma unroll
+      for (int p = 0; p < q; p++) s[q] = fma(v[p], G[(size_t)i * col + i0 + p], s[q]);
+      v[q] = i > r ? -TAU[i] * s[q] : t[i];
+      if (i > r && lane == 0) t[i] = v[q];
     }
+    __syncwarp();
   }
+  for (int c = r + lane; c < col; c += 32) T[transposed ? r + (size_t)c * ldt : c + (size_t)r * ldt] = t[c];
 }
 
 // tile_dlarft (tile_kernel.c:368-437) with 2 <= block < col: couples the
@@ -276,38 +362,85 @@ __global__ void __launch_bounds__(kThreads) k_dlarft_block(int row, int col, int
   }
 }
 
+// One column of W = Y^T a: out[r] = [first[r] +] sum_{q >= (lower ? r : 0)}
+// Y(q, r) a(q), r < Y_col, by the CTA: a warp takes four r at a time.
+__device__ void column_yta(int row, int Y_col, const double* Y, int ldy, const double* a, const double* first,
+                           double* out, bool lower) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  for (int r0 = 4 * warp; r0 < Y_col; r0 += 4 * kWarps) {
+    double s[4] = {0.0, 0.0, 0.0, 0.0};
+    for (int q = (lower ? r0 : 0) + lane; q < row; q += 32) {
+      const double x = a[q];
+#pragma unroll
+      for (int p = 0; p < 4; p++)
+        if (r0 + p < Y_col && (!lower || q >= r0 + p)) s[p] = fma(x, Y[q + (size_t)(r0 + p) * ldy], s[p]);
+    }
+    warp_sums_fixed(s);
+#pragma unroll
+    for (int p = 0; p < 4; p++)
+      if (r0 + p < Y_col && lane == p) out[r0 + p] = (first ? first[r0 + p] : 0.0) + s[p];
+  }
+  __syncthreads();
+}
+
+// One column of a product with n terms: f(r, k) x[k] summed over k < terms(r),
+// by the CTA, rows r < rows; done(r, sum).  Up to kThreads / 32 splits of the
+// sum where there are few rows.  part: kThreads shared doubles.
+template <class F, class N, class Done>
+__device__ void column_product(int rows, N terms, F f, Done done, double* part) {
+  int P = (rows + 31) & ~31;
+  if (P > kThreads) P = kThreads;
+  const int S = kThreads / P, r1 = threadIdx.x % P, s = threadIdx.x / P;
+  for (int rb = 0; rb < rows; rb += P) {
+    const int r = rb + r1;
+    double v = 0.0;
+    if (r < rows && s < S) {
+      const int n = terms(r);
+#pragma unroll 4
+      for (int k = s; k < n; k += S) v = f(r, k, v);
+    }
+    part[threadIdx.x] = v;
+    __syncthreads();
+    if (s == 0 && r < rows) {
+      for (int q = 1; q < S; q++) v += part[q * P + r1];
+      done(r, v);
+    }
+    __syncthreads();
+  }
+}
+
+// W = T w (T lower as stored; transT: the transpose of T's lower part).
+__device__ void column_tw(int n, const double* T, int ldt, int transT, const double* w, double* out, double* part) {
+  if (transT)   // T(q, r), q >= r
+    column_product(n, [=](int r) { return n - r; },
+                   [=](int r, int k, double v) { return fma(T[r + k + (size_t)r * ldt], w[r + k], v); },
+                   [=](int r, double v) { out[r] = v; }, part);
+  else
+    column_product(n, [=](int r) { return r + 1; },
+                   [=](int r, int k, double v) { return fma(T[r + (size_t)k * ldt], w[k], v); },
+                   [=](int r, double v) { out[r] = v; }, part);
+}
+
 // tile_sub_dlarfb (tile_kernel.c:264-311): A (row x A_col) <- A - Y T' (Y^T A)
 // with Y lower (row x row, stored diagonal) for the product and Y's first
-// Y_col columns as stored for the update; T' = T (lower) or, with transT, the
-// transpose of T's lower part (tile_return_dlarfb, tile_kernel.c:501-601).
-// D, D2: Y_col x A_col global scratch.
+// Y_col columns as stored for the update (lower: not above the diagonal); T' =
+// T (lower) or, with transT, the transpose of T's lower part
+// (tile_return_dlarfb, tile_kernel.c:501-601).  The columns of A are
+// independent: each block takes columns blockIdx.x, + gridDim.x, ....  D, D2:
+// Y_col x A_col global scratch.
 __global__ void __launch_bounds__(kThreads) k_sub_dlarfb(int row, int Y_col, int A_col, const double* Y,
                                                           int ldy, const double* T, int ldt, double* A, int lda,
-                                                          double* D, double* D2, int transT) {
-  const int tid = threadIdx.x;
-  for (int e = tid; e < Y_col * A_col; e += kThreads) {
-    const int r = e % Y_col, c = e / Y_col;
-    double s = 0.0;
-    for (int q = r; q < row; q++) s = fma(Y[q + (size_t)r * ldy], A[q + (size_t)c * lda], s);
-    D[r + (size_t)c * Y_col] = s;
-  }
-  __syncthreads();
-  for (int e = tid; e < Y_col * A_col; e += kThreads) {
-    const int r = e % Y_col, c = e / Y_col;
-    double s = 0.0;
-    if (transT) {
-      for (int q = r; q < Y_col; q++) s = fma(T[q + (size_t)r * ldt], D[q + (size_t)c * Y_col], s);
-    } else {
-      for (int q = 0; q <= r; q++) s = fma(T[r + (size_t)q * ldt], D[q + (size_t)c * Y_col], s);
-    }
-    D2[r + (size_t)c * Y_col] = s;
-  }
-  __syncthreads();
-  for (int e = tid; e < row * A_col; e += kThreads) {
-    const int r = e % row, c = e / row;
-    double s = 0.0;
-    for (int q = 0; q < Y_col; q++) s = fma(Y[r + (size_t)q * ldy], D2[q + (size_t)c * Y_col], s);
-    A[r + (size_t)c * lda] -= s;
+                                                          double* D, double* D2, int transT, int lower) {
+  __shared__ double part[kThreads];
+  for (int c = blockIdx.x; c < A_col; c += gridDim.x) {
+    double* a = A + (size_t)c * lda;
+    double* d = D + (size_t)c * Y_col;
+    double* d2 = D2 + (size_t)c * Y_col;
+    column_yta(row, Y_col, Y, ldy, a, nullptr, d, true);
+    column_tw(Y_col, T, ldt, transT, d, d2, part);
+    column_product(row, [=](int q) { return lower && q + 1 < Y_col ? q + 1 : Y_col; },
+                   [=](int q, int r, double v) { return fma(Y[q + (size_t)r * ldy], d2[r], v); },
+                   [=](int q, double v) { a[q] -= v; }, part);
   }
 }
 
@@ -316,51 +449,33 @@ __global__ void __launch_bounds__(kThreads) k_sub_dlarfb(int row, int Y_col, int
 //   ld over_row); 2: tile_dssrfb_tail (A2 -= Y D from U).
 // Quirk kept: rows Y_col..over_row-1 of A1 are zeroed (A1 -= its own copy).
 // transT: T read transposed (tile_return_dssrfb).  D: over_row x A_col, D2:
-// Y_col x A_col global scratch.
+// Y_col x A_col global scratch.  Columns as in k_sub_dlarfb.
 __global__ void __launch_bounds__(kThreads) k_sub_dssrfb(int over_row, int under_row, int Y_col, int A_col,
                                                           const double* Y, int ldy, const double* T, int ldt,
                                                           double* A1, int lda1, double* A2, int lda2, double* D,
                                                           double* D2, double* U, int part, int transT) {
-  const int tid = threadIdx.x;
-  if (part != 2) {
-    for (int e = tid; e < over_row * A_col; e += kThreads) {
-      const int r = e % over_row, c = e / over_row;
-      double d = A1[r + (size_t)c * lda1];
-      if (r < Y_col) {
-        double s = 0.0;
-        for (int q = 0; q < under_row; q++) s = fma(Y[q + (size_t)r * ldy], A2[q + (size_t)c * lda2], s);
-        d += s;
+  __shared__ double sums[kThreads];
+  for (int c = blockIdx.x; c < A_col; c += gridDim.x) {
+    double* a1 = A1 + (size_t)c * lda1;
+    double* a2 = A2 + (size_t)c * lda2;
+    const double* w = U + (size_t)c * over_row;
+    if (part != 2) {
+      double* d = D + (size_t)c * over_row;
+      double* d2 = D2 + (size_t)c * Y_col;
+      column_yta(under_row, min(Y_col, over_row), Y, ldy, a2, a1, d, false);
+      column_tw(Y_col, T, ldt, transT, d, d2, sums);
+      for (int r = threadIdx.x; r < over_row; r += kThreads) {
+        const double v = r < Y_col ? d2[r] : a1[r];
+        a1[r] -= v;
+        if (part == 1) U[r + (size_t)c * over_row] = v;
       }
-      D[r + (size_t)c * over_row] = d;
+      if (part == 1) continue;
+      __syncthreads();
+      w = d2;
     }
-    __syncthreads();
-    for (int e = tid; e < Y_col * A_col; e += kThreads) {
-      const int r = e % Y_col, c = e / Y_col;
-      double s = 0.0;
-      if (transT) {
-        for (int q = r; q < Y_col; q++) s = fma(T[q + (size_t)r * ldt], D[q + (size_t)c * over_row], s);
-      } else {
-        for (int q = 0; q <= r; q++) s = fma(T[r + (size_t)q * ldt], D[q + (size_t)c * over_row], s);
-      }
-      D2[r + (size_t)c * Y_col] = s;
-    }
-    __syncthreads();
-    for (int e = tid; e < over_row * A_col; e += kThreads) {
-      const int r = e % over_row, c = e / over_row;
-      const double d = (r < Y_col) ? D2[r + (size_t)c * Y_col] : D[r + (size_t)c * over_row];
-      A1[r + (size_t)c * lda1] -= d;
-      if (part == 1) U[r + (size_t)c * over_row] = d;
-    }
-    if (part == 1) return;
-    __syncthreads();
-  }
-  const double* W = (part == 2) ? U : D2;
-  const int ldw = (part == 2) ? over_row : Y_col;
-  for (int e = tid; e < under_row * A_col; e += kThreads) {
-    const int r = e % under_row, c = e / under_row;
-    double s = 0.0;
-    for (int q = 0; q < Y_col; q++) s = fma(Y[r + (size_t)q * ldy], W[q + (size_t)c * ldw], s);
-    A2[r + (size_t)c * lda2] -= s;
+    column_product(under_row, [=](int) { return Y_col; },
+                   [=](int q, int r, double v) { return fma(Y[q + (size_t)r * ldy], w[r], v); },
+                   [=](int q, double v) { a2[q] -= v; }, sums);
   }
 }
 
@@ -492,26 +607,81 @@ class Call {
 };
 
 // Launch helpers on device pointers (all sizes already validated).
-void sub_dgeqr2(cudaStream_t s, int row, int col, double* A, int lda, double* TAU, double* Y) {
-  k_sub_dgeqr2<<<1, kThreads, (size_t)(col > 0 ? col : 1) * sizeof(double), s>>>(row, col, A, lda, TAU, Y);
+template <class Kernel>
+void opt_in(Kernel k, size_t smem) {
+  if (smem > 48 * 1024) cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
 }
-void sub_dtsqr2(cudaStream_t s, int row, int col, double* A1, int lda1, double* A2, int lda2, double* TAU) {
-  k_sub_dtsqr2<<<1, kThreads, (size_t)(col > 0 ? col : 1) * sizeof(double), s>>>(row, col, A1, lda1, A2, lda2,
-                                                                                   TAU);
-}
+int column_blocks(int cols) { return cols < 2 * dag_sm_count() ? cols : 2 * dag_sm_count(); }
+
+// G: col x col scratch.
 void sub_dlarft(cudaStream_t s, int row, int col, const double* Y, int lda, const double* TAU, double* T, int ldt,
-                double* G, int transpose_out) {
-  k_sub_dlarft<<<1, kThreads, 0, s>>>(row, col, Y, lda, TAU, T, ldt, G, transpose_out);
+                double* G, bool lower = false, bool zero_upper = false, bool transposed = false) {
+  k_gram<<<col, kThreads, 0, s>>>(row, col, Y, lda, G, lower ? 1 : 0);
+  int warps = kWarps;   // t of a block's columns in 48 KiB where that allows it
+  while (warps > 1 && (size_t)warps * col * sizeof(double) > 48 * 1024) warps /= 2;
+  const size_t smem = (size_t)warps * col * sizeof(double);
+  opt_in(k_larft_cols, smem);
+  k_larft_cols<<<(col + warps - 1) / warps, warps * 32, smem, s>>>(col, G, TAU, T, ldt, zero_upper ? 1 : 0,
+                                                                   transposed ? 1 : 0);
 }
 void sub_dlarfb(cudaStream_t s, int row, int Y_col, int A_col, const double* Y, int ldy, const double* T, int ldt,
-                double* A, int lda, double* D, double* D2, int transT) {
-  k_sub_dlarfb<<<1, kThreads, 0, s>>>(row, Y_col, A_col, Y, ldy, T, ldt, A, lda, D, D2, transT);
+                double* A, int lda, double* D, double* D2, int transT, bool lower = false) {
+  k_sub_dlarfb<<<column_blocks(A_col), kThreads, 0, s>>>(row, Y_col, A_col, Y, ldy, T, ldt, A, lda, D, D2, transT,
+                                                         lower ? 1 : 0);
 }
 void sub_dssrfb(cudaStream_t s, int over_row, int under_row, int Y_col, int A_col, const double* Y, int ldy,
                 const double* T, int ldt, double* A1, int lda1, double* A2, int lda2, double* D, double* D2,
                 double* U, int part, int transT) {
-  k_sub_dssrfb<<<1, kThreads, 0, s>>>(over_row, under_row, Y_col, A_col, Y, ldy, T, ldt, A1, lda1, A2, lda2, D,
-                                     D2, U, part, transT);
+  k_sub_dssrfb<<<column_blocks(A_col), kThreads, 0, s>>>(over_row, under_row, Y_col, A_col, Y, ldy, T, ldt, A1, lda1,
+                                                        A2, lda2, D, D2, U, part, transT);
+}
+// Scratch of the panels wider than one column loop: T and G of a loop's
+// columns, and D, D2 of their application to the rest.
+size_t panel_scratch(int col) { return 2 * (size_t)kMaxW * kMaxW + 2 * (size_t)kMaxW * col; }
+
+// tile_sub_dgeqr2: panels of at most kMaxW columns in shared memory, each
+// applied to the columns right of it; taller ones than fit go column by
+// column through global memory (k_sub_dgeqr2).
+void sub_dgeqr2(cudaStream_t s, int row, int col, double* A, int lda, double* TAU, double* Y, double* work) {
+  double *T = work, *G = T + kMaxW * kMaxW, *D = G + kMaxW * kMaxW, *D2 = D + (size_t)kMaxW * col;
+  const int cw = panel_cols(row);
+  if (cw < 1) {
+    k_sub_dgeqr2<<<1, kThreads, (size_t)col * sizeof(double), s>>>(row, col, A, lda, TAU, Y);
+    return;
+  }
+  opt_in(k_panel<false>, kPanelSmem);
+  for (int j = 0; j < col; j += cw) {
+    const int jb = col - j < cw ? col - j : cw, rows = row - j, rest = col - j - jb;
+    double* Aj = A + j + (size_t)j * lda;
+    double* Yj = Y + j + (size_t)j * lda;
+    k_panel<false><<<1, kThreads, ((size_t)rows * jb + kPanelExtra) * sizeof(double), s>>>(rows, jb, nullptr, 0, Aj,
+                                                                                          lda, TAU + j, Yj);
+    if (rest == 0) break;
+    sub_dlarft(s, rows, jb, Yj, lda, TAU + j, T, kMaxW, G, true, true);
+    sub_dlarfb(s, rows, jb, rest, Yj, lda, T, kMaxW, Aj + (size_t)jb * lda, lda, D, D2, 0, true);
+  }
+}
+// tile_sub_dtsqr2, in the same way.
+void sub_dtsqr2(cudaStream_t s, int row, int col, double* A1, int lda1, double* A2, int lda2, double* TAU,
+                double* work) {
+  double *T = work, *G = T + kMaxW * kMaxW, *D = G + kMaxW * kMaxW, *D2 = D + (size_t)kMaxW * col;
+  const int cw = panel_cols(row);
+  if (cw < 1) {
+    k_sub_dtsqr2<<<1, kThreads, (size_t)col * sizeof(double), s>>>(row, col, A1, lda1, A2, lda2, TAU);
+    return;
+  }
+  opt_in(k_panel<true>, kPanelSmem);
+  for (int j = 0; j < col; j += cw) {
+    const int jb = col - j < cw ? col - j : cw, rest = col - j - jb;
+    double* A1j = A1 + j + (size_t)j * lda1;
+    double* A2j = A2 + (size_t)j * lda2;
+    k_panel<true><<<1, kThreads, ((size_t)row * jb + kPanelExtra) * sizeof(double), s>>>(row, jb, A1j, lda1, A2j,
+                                                                                        lda2, TAU + j, nullptr);
+    if (rest == 0) break;
+    sub_dlarft(s, row, jb, A2j, lda2, TAU + j, T, kMaxW, G, false, true);
+    sub_dssrfb(s, jb, row, jb, rest, A2j, lda2, T, kMaxW, A1j + (size_t)jb * lda1, lda1, A2j + (size_t)jb * lda2,
+               lda2, D, D2, nullptr, 0, 0);
+  }
 }
 
 }  // namespace tk
@@ -541,8 +711,10 @@ void tile_sub_dgeqr2(const int row, const int col, double* A, const int lda, dou
   double* dA = call.arg(A, extent(lda, row, col), true);
   double* dT = call.arg(TAU, col, true);
   double* dY = call.arg(Y, extent(lda, row, col), true);
-  if (!call.bind()) return;
-  hqr::tk::sub_dgeqr2(call.stream(), row, col, call.view(A, dA), lda, call.view(TAU, dT), call.view(Y, dY));
+  const size_t w = call.scratch(hqr::tk::panel_scratch(col));
+  double* base = call.bind();
+  if (!base) return;
+  hqr::tk::sub_dgeqr2(call.stream(), row, col, call.view(A, dA), lda, call.view(TAU, dT), call.view(Y, dY), base + w);
   call.launched();
 }
 
@@ -555,9 +727,11 @@ void tile_sub_dtsqr2(const int row, const int col, double* A1, const int lda1, d
   double* d1 = call.arg(A1, extent(lda1, col, col), true);
   double* d2 = call.arg(A2, extent(lda2, row, col), true);
   double* dt = call.arg(TAU, col, true);
-  if (!call.bind()) return;
+  const size_t w = call.scratch(hqr::tk::panel_scratch(col));
+  double* base = call.bind();
+  if (!base) return;
   hqr::tk::sub_dtsqr2(call.stream(), row, col, call.view(A1, d1), lda1, call.view(A2, d2), lda2,
-                      call.view(TAU, dt));
+                      call.view(TAU, dt), base + w);
   call.launched();
 }
 
@@ -574,7 +748,7 @@ void tile_sub_dlarft(const int row, const int col, const double* Y, const int ld
   double* base = call.bind();
   if (!base) return;
   hqr::tk::sub_dlarft(call.stream(), row, col, call.view(Y, dy), lda, call.view(TAU, dtau), call.view(T, dT), ldt,
-                      base + g, 0);
+                      base + g);
   call.launched();
 }
 
@@ -630,6 +804,7 @@ void tile_dgeqrt(const int row, const int col, const int block, double* A, const
   double* dT = call.arg(T, extent(ldt, col, col), true);
   const size_t g = call.scratch((size_t)col * col);
   const size_t d = call.scratch((size_t)row * col), d2 = call.scratch((size_t)row * col);
+  const size_t w = call.scratch(hqr::tk::panel_scratch(col));
   double* base = call.bind();
   if (!base) return;
   A = call.view(A, dA);
@@ -639,13 +814,13 @@ void tile_dgeqrt(const int row, const int col, const int block, double* A, const
   cudaStream_t s = call.stream();
   int i;
   for (i = 0; i < col - block; i += block) {
-    hqr::tk::sub_dgeqr2(s, row - i, block, A + i * lda + i, lda, TAU + i, Y + i * lda + i);
-    hqr::tk::sub_dlarft(s, row - i, block, Y + i * lda + i, lda, TAU + i, T + i * ldt + i, ldt, base + g, 0);
+    hqr::tk::sub_dgeqr2(s, row - i, block, A + i * lda + i, lda, TAU + i, Y + i * lda + i, base + w);
+    hqr::tk::sub_dlarft(s, row - i, block, Y + i * lda + i, lda, TAU + i, T + i * ldt + i, ldt, base + g);
     hqr::tk::sub_dlarfb(s, row - i, block, col - i - block, Y + i * lda + i, lda, T + i * ldt + i, ldt,
                         A + (i + block) * lda + i, lda, base + d, base + d2, 0);
   }
-  hqr::tk::sub_dgeqr2(s, row - i, col - i, A + i * lda + i, lda, TAU + i, Y + i * lda + i);
-  hqr::tk::sub_dlarft(s, row - i, col - i, Y + i * lda + i, lda, TAU + i, T + i * ldt + i, ldt, base + g, 0);
+  hqr::tk::sub_dgeqr2(s, row - i, col - i, A + i * lda + i, lda, TAU + i, Y + i * lda + i, base + w);
+  hqr::tk::sub_dlarft(s, row - i, col - i, Y + i * lda + i, lda, TAU + i, T + i * ldt + i, ldt, base + g);
   call.launched();
 }
 
@@ -661,6 +836,7 @@ void tile_dtsqrt(const int row, const int col, const int block, double* A1, cons
   double* dT = call.arg(T, extent(ldt, col, col), true);
   const size_t g = call.scratch((size_t)col * col);
   const size_t d = call.scratch((size_t)block * col), dd = call.scratch((size_t)block * col);
+  const size_t w = call.scratch(hqr::tk::panel_scratch(col));
   double* base = call.bind();
   if (!base) return;
   A1 = call.view(A1, d1);
@@ -670,20 +846,20 @@ void tile_dtsqrt(const int row, const int col, const int block, double* A1, cons
   cudaStream_t s = call.stream();
   int i;
   for (i = 0; i < col - block; i += block) {
-    hqr::tk::sub_dtsqr2(s, row, block, A1 + i + i * lda1, lda1, A2 + i * lda2, lda2, TAU + i);
-    hqr::tk::sub_dlarft(s, row, block, A2 + i * lda2, lda2, TAU + i, T + i * ldt + i, ldt, base + g, 0);
+    hqr::tk::sub_dtsqr2(s, row, block, A1 + i + i * lda1, lda1, A2 + i * lda2, lda2, TAU + i, base + w);
+    hqr::tk::sub_dlarft(s, row, block, A2 + i * lda2, lda2, TAU + i, T + i * ldt + i, ldt, base + g);
     hqr::tk::sub_dssrfb(s, block, row, block, col - i - block, A2 + i * lda2, lda2, T + i + i * ldt, ldt,
                         A1 + i + (i + block) * lda1, lda1, A2 + (i + block) * lda2, lda2, base + d, base + dd,
                         nullptr, 0, 0);
   }
   if (col % block > 0) {
     i = block * (col / block);
-    hqr::tk::sub_dtsqr2(s, row, col % block, A1 + i + i * lda1, lda1, A2 + i * lda2, lda2, TAU + i);
-    hqr::tk::sub_dlarft(s, row, col % block, A2 + i * lda2, lda2, TAU + i, T + i * ldt + i, ldt, base + g, 0);
+    hqr::tk::sub_dtsqr2(s, row, col % block, A1 + i + i * lda1, lda1, A2 + i * lda2, lda2, TAU + i, base + w);
+    hqr::tk::sub_dlarft(s, row, col % block, A2 + i * lda2, lda2, TAU + i, T + i * ldt + i, ldt, base + g);
   } else {
     i = col - block;
-    hqr::tk::sub_dtsqr2(s, row, block, A1 + i + i * lda1, lda1, A2 + i * lda2, lda2, TAU + i);
-    hqr::tk::sub_dlarft(s, row, block, A2 + i * lda2, lda2, TAU + i, T + i * ldt + i, ldt, base + g, 0);
+    hqr::tk::sub_dtsqr2(s, row, block, A1 + i + i * lda1, lda1, A2 + i * lda2, lda2, TAU + i, base + w);
+    hqr::tk::sub_dlarft(s, row, block, A2 + i * lda2, lda2, TAU + i, T + i * ldt + i, ldt, base + g);
   }
   call.launched();
 }
@@ -801,21 +977,11 @@ void tile_return_dlarft(const int row, const int col, const double* Y, const int
   double* dy = call.arg(Y, extent(lda, row, col), false);
   double* dtau = call.arg(TAU, col, false);
   double* dT = call.arg(T, extent(ldt, col, col), true);
-  const size_t g = call.scratch((size_t)col * col), ts = call.scratch((size_t)col * col);
+  const size_t g = call.scratch((size_t)col * col);
   double* base = call.bind();
   if (!base) return;
-  cudaStream_t s = call.stream();
-  if (cudaMemsetAsync(base + ts, 0, (size_t)col * col * sizeof(double), s) != cudaSuccess) {
-    call.launched();
-    return;
-  }
-  hqr::tk::sub_dlarft(s, row, col, call.view(Y, dy), lda, call.view(TAU, dtau), base + ts, col, base + g, 1);
-  // copy the upper triangle (with the diagonal) into T
-  T = call.view(T, dT);
-  for (int c = 0; c < col; c++)
-    if (cudaMemcpyAsync(T + (size_t)c * ldt, base + ts + (size_t)c * col, (size_t)(c + 1) * sizeof(double),
-                        cudaMemcpyDeviceToDevice, s) != cudaSuccess)
-      break;
+  hqr::tk::sub_dlarft(call.stream(), row, col, call.view(Y, dy), lda, call.view(TAU, dtau), call.view(T, dT), ldt,
+                      base + g, false, true, true);
   call.launched();
 }
 
