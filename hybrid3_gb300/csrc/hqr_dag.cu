@@ -9,6 +9,17 @@
 
 namespace hqr {
 
+// Task ids of the plain FP64 factorization without trailing-update tasks, and
+// the bytes of scratch that hqr_geqrf_noalloc carves for n_ids ids.
+static size_t coarse_task_ids(const Geometry& g) {
+  return (size_t)g.steps * g.MT * (g.NB / g.w) + (size_t)g.steps * g.NT * g.MT * g.NC;
+}
+size_t external_bytes(const Geometry& g, size_t n_ids) {
+  auto round256 = [](size_t b) { return (b + 255) & ~size_t(255); };
+  return round256((size_t)g.M * g.N * sizeof(double)) + 3 * round256(n_ids * sizeof(int)) +
+         round256(kExternalCtlBytes) + round256(kExternalStatsBytes);
+}
+
 int make_geometry(long M, long N, int NB, int IB, Geometry* g, size_t smem_limit) {
   if (NB < 16 || NB > kMaxNB || NB % 16 != 0) return HQR_ERR_UNSUPPORTED;
   if (M <= 0 || N <= 0 || M % NB != 0 || N % NB != 0) return HQR_ERR_INVALID;
@@ -58,7 +69,6 @@ int dag_workspace_reserve(DagWorkspace* ws, size_t n_ids) {
   if (ws->cap_ids >= n_ids && ws->ctl) return HQR_OK;
   dag_workspace_free(ws);
   if (cudaMalloc(&ws->cnt, n_ids * sizeof(int)) != cudaSuccess) return HQR_ERR_NOMEM;
-  if (cudaMalloc(&ws->flag, n_ids * sizeof(int)) != cudaSuccess) return HQR_ERR_NOMEM;
   if (cudaMalloc(&ws->qhi, n_ids * sizeof(int)) != cudaSuccess) return HQR_ERR_NOMEM;
   if (cudaMalloc(&ws->qlo, n_ids * sizeof(int)) != cudaSuccess) return HQR_ERR_NOMEM;
   if (cudaMalloc(&ws->ctl, kCtlWords * sizeof(unsigned)) != cudaSuccess) return HQR_ERR_NOMEM;
@@ -71,7 +81,6 @@ int dag_workspace_reserve(DagWorkspace* ws, size_t n_ids) {
 
 void dag_workspace_free(DagWorkspace* ws) {
   if (ws->cnt) cudaFree(ws->cnt);
-  if (ws->flag) cudaFree(ws->flag);
   if (ws->qhi) cudaFree(ws->qhi);
   if (ws->qlo) cudaFree(ws->qlo);
   if (ws->ctl) cudaFree(ws->ctl);
@@ -150,7 +159,6 @@ static int run_dag(DagParams& p, DagWorkspace* ws, const Geometry& g, cudaStream
   int rc = dag_workspace_reserve(ws, (size_t)p.n_ids);
   if (rc != HQR_OK) return rc;
   p.cnt = ws->cnt;
-  p.tsflag = ws->flag;
   p.qhi = ws->qhi;
   p.qlo = ws->qlo;
   p.ctl = ws->ctl;
@@ -169,9 +177,34 @@ static int run_dag(DagParams& p, DagWorkspace* ws, const Geometry& g, cudaStream
   return p.oz_p32 ? launch_exec<true, 4, true>(p, g, stream) : launch_exec<true, 4>(p, g, stream);
 }
 
-// Update tiles left in a step below which the factorization's panel blocks
-// run in phases (DagParams::ts_split).
-constexpr long long kPhasedWork = 6000;
+// The steps from which on a flat-tree factorization cuts its panel blocks'
+// trailing updates into tasks of their own: those whose panel chain, not their
+// update work, sets the pace, that is with at most `tiles` update tiles ((NT -
+// i - 1) (MT - i - 1)) left.  Before them the additional tasks cost more than
+// the shorter chain gains.  Measured, against whole panel blocks: FP64 n =
+// 2048, NB 256: factorization 73 -> 38 ms; n = 4096: 155 -> 118 ms; split n =
+// 3072 (against blocks that released their dependents in phases): QR + Q 35.7
+// -> 28.4 ms; split n = 16384 unchanged.
+struct FineSteps {
+  int from = 0;
+  long long ids = 0, tasks = 0;
+};
+constexpr long long kFineTilesSplit = 6000, kFineTilesFp64 = 600;
+static FineSteps fine_steps(const Geometry& g, bool split) {
+  FineSteps f;
+  const long long nblk = g.NB / g.w, tiles = split ? kFineTilesSplit : kFineTilesFp64;
+  while (f.from < g.steps && (long long)(g.NT - f.from - 1) * (g.MT - f.from - 1) > tiles) f.from++;
+  if (nblk < 2) return f;
+  f.ids = (long long)(g.steps - f.from) * g.MT * nblk * nblk;
+  for (int i = f.from; i < g.steps; i++) f.tasks += (g.MT - i) * nblk * (nblk - 1) / 2;
+  // the allocation-free entry point has the same tasks, hence the same
+  // rounding: where its scratch holds the factorization without these ids but
+  // not with them, neither has them
+  const size_t plain = external_bytes(g, coarse_task_ids(g));
+  const bool squeezed = plain <= kNoAllocScratchBytes && external_bytes(g, coarse_task_ids(g) + f.ids) > kNoAllocScratchBytes;
+  if ((!split && squeezed) || (long long)coarse_task_ids(g) + f.ids > 0x3fffffffLL) f.ids = f.tasks = 0;
+  return f;
+}
 
 // 64-column chunks per split update task, run one after the other.  Two (a
 // whole 128-column tile) halve the number of update tasks and with them the
@@ -236,23 +269,14 @@ int launch_factor(const Geometry& g, DagWorkspace* ws, double* dA, double* dT, d
   p.prep = p.oz;
   p.nblk = g.NB / g.w;
   set_tree(p, g, tw);
-  // split precision, flat tree: panel blocks release their panel dependents
-  // in phases (the first trailing column block is then w wide, which changes
-  // the rounding of the FP64 panels' trailing sums, so FP64 plans keep the
-  // whole-block releases and their results)
-  p.ts_split = (p.tree == 0 && p.oz) ? 1 : 0;
-  // only in the steps whose panel chain, not their update work, sets the
-  // pace: few update tiles left ((NT - i - 1) (MT - i - 1) at most
-  // kPhasedWork); before them the phases' waits and narrower first column
-  // block cost more than the shorter chain gains
-  p.ts_split_from = 0;
-  while (p.ts_split_from < g.steps &&
-         (long long)(g.NT - p.ts_split_from - 1) * (g.MT - p.ts_split_from - 1) > kPhasedWork)
-    p.ts_split_from++;
+  const FineSteps fine = p.tree == 0 ? fine_steps(g, p.oz != 0) : FineSteps{};
+  p.fine_from = fine.from;
+  p.fine_ids = (int)fine.ids;
   // tasks: per step i, nblk inner blocks of each of the MT-i panel tiles [+ one
   // OZPREP per panel tile] + NC*(NT-1-i)*(MT-i) updates; a tree adds per merge
-  // nblk blocks [+ one OZPREP] + NC*(NT-1-i) merge updates
-  long long n = 0;
+  // nblk blocks [+ one OZPREP] + NC*(NT-1-i) merge updates; a fine step nblk
+  // (nblk - 1) / 2 trailing updates per panel tile
+  long long n = fine.tasks;
   for (int i = 0; i < g.steps; i++) {
     const long long m = merges_of_step(p, i);
     n += (long long)(g.MT - i) * (p.nblk + (p.prep ? 1 : 0)) + (long long)p.NC * (g.NT - 1 - i) * (g.MT - i);
@@ -547,9 +571,7 @@ size_t tree_slots(const Geometry& g, int S) {
   return (size_t)g.steps * ((g.MT + S - 1) / S);
 }
 
-size_t factor_task_ids(const Geometry& g) {
-  return (size_t)g.steps * g.MT * (g.NB / g.w) + (size_t)g.steps * g.NT * g.MT * g.NC;
-}
+size_t factor_task_ids(const Geometry& g) { return coarse_task_ids(g) + (size_t)fine_steps(g, false).ids; }
 
 int launch_factor_external(const Geometry& g, const ExternalScratch& x, double* dA, double* dTAU,
                            long long timeout_ns, cudaStream_t stream) {
@@ -566,8 +588,11 @@ int launch_factor_external(const Geometry& g, const ExternalScratch& x, double* 
   p.nblk = g.NB / g.w;
   p.sh = shape_of(g);
   p.sp = SmemPlan::make(p.sh);
+  const FineSteps fine = fine_steps(g, false);
+  p.fine_from = fine.from;
+  p.fine_ids = (int)fine.ids;
   p.n_ids = (int)factor_task_ids(g);
-  long long n = 0;
+  long long n = fine.tasks;
   for (int i = 0; i < g.steps; i++)
     n += (long long)(g.MT - i) * p.nblk + (long long)g.NC * (g.NT - 1 - i) * (g.MT - i);
   p.n_tasks = (int)n;

@@ -57,7 +57,10 @@ __host__ __device__ __forceinline__ bool applies_h(int mode) { return mode == kM
 enum TaskType : int {
   kGEQRT = 0, kTSQRT = 1, kLARFB = 2, kSSRFB = 3, kTBUILD = 4, kOZPREP = 5, kNumTypes = 6,
   // the merges of a domain tree (counted with TSQRT, OZPREP and SSRFB)
-  kTTQRT = 6, kTTPREP = 7, kTTMQR = 8
+  kTTQRT = 6, kTTPREP = 7, kTTMQR = 8,
+  // one column block of a panel block's trailing update (DagParams::fine_ids;
+  // its cycles are counted with GEQRT / TSQRT)
+  kTRAIL = 9
 };
 __host__ __device__ __forceinline__ int stat_slot(int type) {
   return type == kTTQRT ? kTSQRT : type == kTTPREP ? kOZPREP : type == kTTMQR ? kSSRFB : type;
@@ -107,15 +110,11 @@ struct DagParams {
   double* TAU;
   double* C;        // target of the update tasks (A itself when factoring)
   int* cnt;         // dependency counters, one per task id
-  // Factorization with the flat tree (ts_split): a panel block (GEQRT or
-  // TSQRT inner block b of tile k at step i) releases the same block of the
-  // tile below once its reflectors are stored, and the next block of its
-  // own tile once the next block's w columns are updated; tsflag[its id]
-  // is set when its whole trailing update is done, which the later blocks
-  // that share those columns or R's rows wait for (bounded) before theirs.
-  int ts_split;
-  int ts_split_from;   // the first step whose panel blocks use the phases
-  int* tsflag;
+  // Factorization with the flat tree, fine_ids > 0: in the steps from
+  // fine_from on, a panel block (GEQRT or TSQRT inner block b of tile k) is its
+  // column loop only; its trailing update is one task per later w-column block
+  // j of the tile (fine_ids task ids).
+  int fine_from, fine_ids;
   int* qhi;         // ready FIFOs, capacity n_ids each
   int* qlo;
   unsigned* ctl;
@@ -168,6 +167,7 @@ __host__ __device__ __forceinline__ bool is_top(const DagParams& p, int i, int k
 //   merge  (i, d, b)     : M0 + (i*dmax + d)*nblk + b            (1 <= d < domains)
 //   merge prep (i, d)    : Q0 + i*dmax + d     (split precision)
 //   merge update (i, j, d, c): X0 + ((i*J + j)*dmax + d)*NC + c
+//   trailing (i, k, b, j): Y0 + (((i - fine_from)*MT + k)*nblk + b)*nblk + j   (j > b, i >= fine_from)
 __host__ __device__ __forceinline__ int panel_id(const DagParams& p, int i, int k, int b = 0) {
   return (i * p.MT + k) * p.nblk + b;
 }
@@ -201,9 +201,16 @@ __host__ __device__ __forceinline__ int ttmqr_base(const DagParams& p) {
 __host__ __device__ __forceinline__ int ttmqr_id(const DagParams& p, int i, int j, int d, int c) {
   return ttmqr_base(p) + ((i * p.J + j) * p.dmax + d) * p.NC + c;
 }
-__host__ __device__ __forceinline__ int id_end(const DagParams& p) {
+__host__ __device__ __forceinline__ int trail_base(const DagParams& p) {
   return ttmqr_base(p) + p.steps * p.J * p.dmax * p.NC;
 }
+__host__ __device__ __forceinline__ int trail_id(const DagParams& p, int i, int k, int b, int j) {
+  return trail_base(p) + (((i - p.fine_from) * p.MT + k) * p.nblk + b) * p.nblk + j;
+}
+__host__ __device__ __forceinline__ bool fine_step(const DagParams& p, int i) {
+  return p.fine_ids > 0 && i >= p.fine_from;
+}
+__host__ __device__ __forceinline__ int id_end(const DagParams& p) { return trail_base(p) + p.fine_ids; }
 // Compact index of merge (i, d) into T2 / TAU2 / slices2.
 __host__ __device__ __forceinline__ size_t merge_slot(const DagParams& p, int i, int d) {
   return (size_t)i * p.dmax + d;
@@ -214,7 +221,7 @@ __host__ __device__ __forceinline__ size_t panel_slot(int MT, int i, int k) {
 }
 
 struct TaskDesc {
-  int type, i, j, k, c;   // c: column block of an update, inner block of a panel task
+  int type, i, j, k, c;   // c: column block of an update, inner block of a panel task (kTRAIL: j its column block)
 };
 
 __device__ __forceinline__ TaskDesc decode(const DagParams& p, int id) {
@@ -260,7 +267,7 @@ __device__ __forceinline__ TaskDesc decode(const DagParams& p, int id) {
     t.k = dom_top(p, t.i, d);
     t.c = 0;
     t.type = kTTPREP;
-  } else {
+  } else if (id < trail_base(p)) {
     int u = id - ttmqr_base(p);
     t.c = u % p.NC; u /= p.NC;
     const int d = u % p.dmax; u /= p.dmax;
@@ -268,6 +275,13 @@ __device__ __forceinline__ TaskDesc decode(const DagParams& p, int id) {
     t.i = u / p.J;
     t.k = dom_top(p, t.i, d);
     t.type = kTTMQR;
+  } else {
+    int u = id - trail_base(p);
+    t.j = u % p.nblk; u /= p.nblk;
+    t.c = u % p.nblk; u /= p.nblk;
+    t.k = u % p.MT;
+    t.i = p.fine_from + u / p.MT;
+    t.type = kTRAIL;
   }
   return t;
 }
@@ -281,7 +295,7 @@ __device__ __forceinline__ bool update_valid(const DagParams& p, int i, int j) {
 __device__ __forceinline__ bool is_high_priority(const DagParams& p, int id) {
   const TaskDesc t = decode(p, id);
   if (t.type == kGEQRT || t.type == kTSQRT || t.type == kTBUILD || t.type == kOZPREP ||
-      t.type == kTTQRT || t.type == kTTPREP)
+      t.type == kTTQRT || t.type == kTTPREP || t.type == kTRAIL)
     return true;
   return p.mode == kModeFactor && t.j == t.i + 1;   // look-ahead: next panel column
 }
@@ -398,8 +412,9 @@ __device__ int init_deps(const DagParams& p, int id) {
     const int i = tile / p.MT, k = tile % p.MT;
     if (k >= i && !p.skip_panels) {
       // block 0: the previous step's update of the tile (NC column blocks);
-      // block b > 0: block b - 1 of the same tile; a TSQRT block also waits
-      // for the same block of the tile above (its domain top's rows of R)
+      // block b > 0: block b - 1 of the same tile (in a fine step: its trailing
+      // update of column block b); a TSQRT block also waits for the same block
+      // of the tile above (its domain top's rows of R)
       if (p.mode == kModeFactor)
         deps = (b == 0 ? (i > 0 ? p.NC : 0) : 1) + (is_top(p, i, k) ? 0 : 1);
       else
@@ -432,6 +447,14 @@ __device__ int init_deps(const DagParams& p, int id) {
     const int u = id - ttprep_base(p);
     const int d = u % p.dmax, i = u / p.dmax;
     if (i < p.steps && d >= 1 && d < n_domains(p, i) && !p.skip_panels) deps = 1;
+  } else if (id >= trail_base(p)) {
+    // trailing (i, k, b, j): panel block b of the tile; the earlier block's
+    // update of the same columns; the tile above's update of R's rows
+    int u = id - trail_base(p);
+    const int j = u % p.nblk; u /= p.nblk;
+    const int b = u % p.nblk; u /= p.nblk;
+    const int k = u % p.MT, i = p.fine_from + u / p.MT;
+    if (k >= i && j > b) deps = 1 + (b > 0 ? 1 : 0) + (k > i ? 1 : 0);
   } else {
     // merge update: the merge (unless given), domain d's chain on column j,
     // the previous merge update (domain 0's chain for d = 1)
@@ -451,7 +474,6 @@ __global__ void dag_init_kernel(DagParams p) {
   p.qhi[id] = -1;
   p.qlo[id] = -1;
   p.cnt[id] = init_deps(p, id);
-  if (p.ts_split && id < panel_end(p)) p.tsflag[id] = 0;
 }
 
 __global__ void dag_seed_kernel(DagParams p) {
@@ -577,13 +599,15 @@ __device__ bool release_dependents(const DagParams& p, const TaskDesc& t, int* k
       // the next inner block of this tile; the same block of the tile below in
       // the domain, or, from a domain's last tile, of the domain's merge
       const int d = dom_of(p, t.i, t.k);
-      if (!p.ts_split || t.i < p.ts_split_from) {   // (else the task's phases released these)
-        if (t.c + 1 < p.nblk) release(p, panel_id(p, t.i, t.k, t.c + 1));
-        if (t.k + 1 < dom_end(p, t.i, d))
-          release(p, panel_id(p, t.i, t.k + 1, t.c));
-        else if (n_domains(p, t.i) > 1)
-          release(p, merge_id(p, t.i, d >= 1 ? d : 1, t.c));
+      if (fine_step(p, t.i)) {
+        for (int j = t.c + 1; j < p.nblk; j++) release(p, trail_id(p, t.i, t.k, t.c, j));
+      } else if (t.c + 1 < p.nblk) {
+        release(p, panel_id(p, t.i, t.k, t.c + 1));
       }
+      if (t.k + 1 < dom_end(p, t.i, d))
+        release(p, panel_id(p, t.i, t.k + 1, t.c));
+      else if (n_domains(p, t.i) > 1)
+        release(p, merge_id(p, t.i, d >= 1 ? d : 1, t.c));
       if (t.c + 1 < p.nblk) return true;   // the tile's V, T, TAU are complete after its last block
     }
     if (feeds_prep) {
@@ -594,6 +618,11 @@ __device__ bool release_dependents(const DagParams& p, const TaskDesc& t, int* k
       for (int j = j0; j < j1; j++)
         for (int c = 0; c < p.NC; c++) release(p, update_id(p, t.i, j, t.k, c));
     }
+    return true;
+  }
+  if (t.type == kTRAIL) {
+    release(p, t.j == t.c + 1 ? panel_id(p, t.i, t.k, t.j) : trail_id(p, t.i, t.k, t.c + 1, t.j));
+    if (t.k + 1 < p.MT) release(p, trail_id(p, t.i, t.k + 1, t.c, t.j));
     return true;
   }
   if (t.type == kTTQRT || t.type == kTTPREP) {
@@ -663,64 +692,6 @@ __device__ void task_tbuild(const double* V, const double* tau_g, double* T, boo
 // registers per thread): while one runs a latency-bound panel column loop,
 // the other's update keeps the FP64 pipe busy.
 // OZG: t-groups of the split updates (8: FP64-level; 4: the reduced form).
-// Thread 0: wait (bounded) until panel block `id` has finished its trailing
-// update; false (error word set) when the wait ran out or the DAG failed.
-__device__ bool wait_ts_flag(const DagParams& p, int id) {
-  const uint64_t t0 = global_ns();
-  while (*((volatile const int*)(p.tsflag + id)) == 0) {
-    if (*((volatile const unsigned*)(p.ctl + kErr)) != 0u) return false;
-    if ((long long)(global_ns() - t0) > p.timeout_ns) {
-      atomicOr((int*)(p.ctl + kErr), kErrTimeout);
-      return false;
-    }
-    __nanosleep(64);
-  }
-  return true;
-}
-
-// The phases of a factorization panel block with ts_split (see DagParams):
-// called by every thread of the CTA at the points task_geqrt_blk /
-// task_tsqrt_blk name.  Every wait is on a block that has already released
-// this one (so it is running, past that release) and that waits only on
-// blocks of smaller b or k itself: no cycle, and each wait is bounded.
-// on == false: no phases (the block releases at its end, as without
-// ts_split), and the trailing update keeps its usual column blocks.
-struct PanelPhases {
-  const DagParams* p;
-  int i, k, b;
-  bool on;
-  __device__ int first_cols(int cb, int w) const { return on ? w : cb; }
-  __device__ void publish() const {   // this CTA's writes, then thread 0 releases
-    fence_acq_rel_gpu();
-    __syncthreads();
-  }
-  __device__ void after_panel() const {   // R's diagonal block is final: the tile below's block b
-    if (!on) return;
-    publish();
-    if (threadIdx.x == 0 && k + 1 < p->MT) release(*p, panel_id(*p, i, k + 1, b));
-  }
-  __device__ void before_trailing() const {
-    if (!on) return;
-    if (threadIdx.x == 0) {
-      bool ok = true;
-      if (b > 0) ok = wait_ts_flag(*p, panel_id(*p, i, k, b - 1));   // the same columns, earlier block
-      if (ok && k > i) ok = wait_ts_flag(*p, panel_id(*p, i, k - 1, b));   // R's rows, tile above
-      fence_acq_rel_gpu();   // acquire: their writes are visible
-    }
-    __syncthreads();
-  }
-  __device__ void after_first() const {   // the next block's columns are updated
-    if (!on) return;
-    publish();
-    if (threadIdx.x == 0 && b + 1 < p->nblk) release(*p, panel_id(*p, i, k, b + 1));
-  }
-  __device__ void after_trailing() const {
-    if (!on) return;
-    publish();
-    if (threadIdx.x == 0) atomicExch(p->tsflag + panel_id(*p, i, k, b), 1);
-  }
-};
-
 // P32: the panel blocks compute in FP32 (HQR_PREC_FP32).
 template <bool OZ, bool BATCH = false, int OZG = 8, bool P32 = false>
 __global__ void __launch_bounds__(kThreads, BATCH ? 2 : 1) dag_exec_kernel(DagParams p) {
@@ -785,7 +756,7 @@ __global__ void __launch_bounds__(kThreads, BATCH ? 2 : 1) dag_exec_kernel(DagPa
       case kGEQRT: {   // the diagonal tile or a domain's top tile
         const size_t o = tile_off(t.k, t.i, q.MT, NB);
         task_geqrt_blk<PanelT>(q.A + o, q.T + o, q.TAU + tau_off(t.k, t.i, q.MT, NB), q.sh, smem, q.sp, t.c,
-                               PanelPhases{&q, t.i, t.k, t.c, q.ts_split != 0 && t.i >= q.ts_split_from});
+                               !fine_step(q, t.i));
         break;
       }
       case kTSQRT: {   // R of the domain's top tile over tile (k, i)
@@ -804,6 +775,13 @@ __global__ void __launch_bounds__(kThreads, BATCH ? 2 : 1) dag_exec_kernel(DagPa
         ts_t = q.T2 + slot * tsz;
         ts_tau = q.TAU2 + slot * NB;
         ts_upper = true;
+        break;
+      }
+      case kTRAIL: {
+        const size_t o = tile_off(t.k, t.i, q.MT, NB);
+        if (!BATCH)
+          task_trailing<PanelT>(q.A + tile_off(t.i, t.i, q.MT, NB), t.k > t.i ? q.A + o : nullptr, q.T + o, q.sh,
+                                smem, q.sp, t.c, t.j);
         break;
       }
       case kTBUILD: {
@@ -870,8 +848,7 @@ __global__ void __launch_bounds__(kThreads, BATCH ? 2 : 1) dag_exec_kernel(DagPa
         if (threadIdx.x == 0) atomicOr((int*)(q.ctl + kErr), kErrBadTask);
     }
     if (ts_a1)
-      task_tsqrt_blk<PanelT>(ts_a1, ts_a2, ts_t, ts_tau, q.sh, smem, q.sp, t.c, ts_upper,
-                             PanelPhases{&q, t.i, t.k, t.c, q.ts_split != 0 && t.i >= q.ts_split_from && !ts_upper});
+      task_tsqrt_blk<PanelT>(ts_a1, ts_a2, ts_t, ts_tau, q.sh, smem, q.sp, t.c, ts_upper, !fine_step(q, t.i));
     // Q generation and Q C apply H (M = T), the other modes H^T (M = T^T)
     if (OZ && prep_v)
       task_ozprep(prep_v, prep_tau, prep_g, prep_kind, prep_slices, prep_exps, reinterpret_cast<uint8_t*>(smem),
@@ -888,9 +865,11 @@ __global__ void __launch_bounds__(kThreads, BATCH ? 2 : 1) dag_exec_kernel(DagPa
     fence_acq_rel_gpu();   // release: this task's writes before its dependents' counters
     __syncthreads();
     if (threadIdx.x == 0) {
-      local_cnt[stat_slot(t.type)]++;
+      const int slot = t.type == kTRAIL ? (t.k > t.i ? kTSQRT : kGEQRT) : stat_slot(t.type);
+      const int counted = t.type == kTRAIL ? 0 : 1;   // (GEQRT / TSQRT: one per panel block)
+      local_cnt[slot] += counted;
       const long long c1 = clock64();
-      local_cyc[stat_slot(t.type)] += (unsigned long long)(c1 - c0);
+      local_cyc[slot] += (unsigned long long)(c1 - c0);
       // the control words are read before the releases so that their round
       // trips overlap the releases' atomics
       volatile unsigned* ctl = q.ctl;
@@ -898,13 +877,13 @@ __global__ void __launch_bounds__(kThreads, BATCH ? 2 : 1) dag_exec_kernel(DagPa
       const bool pushed_hi = release_dependents(q, t, &next);
       cont_ok = err_now == 0u && hi_head >= hi_tail && !pushed_hi;
       atomicAdd(q.ctl + kDone, 1u);   // termination count only: no ordering needed
-      local_cnt[kStatSched]++;
+      local_cnt[kStatSched] += counted;
       local_cyc[kStatSched] += (unsigned long long)(clock64() - c1);
     }
   }
   if (threadIdx.x == 0 && p.stats) {
     for (int ty = 0; ty < kNumStats; ty++) {
-      if (local_cnt[ty]) {
+      if (local_cyc[ty]) {
         atomicAdd(p.stats + 2 * ty, local_cnt[ty]);
         atomicAdd(p.stats + 2 * ty + 1, local_cyc[ty]);
       }

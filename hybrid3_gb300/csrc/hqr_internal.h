@@ -65,7 +65,6 @@ int at_times(const double* dA, long M, long N, int NB, const double* dR, long ld
 // Scheduler workspace (dependency counters, queues, control words, stats).
 struct DagWorkspace {
   int* cnt = nullptr;
-  int* flag = nullptr;   // per panel block: its trailing update is done (factorization)
   int* qhi = nullptr;
   int* qlo = nullptr;
   unsigned* ctl = nullptr;
@@ -159,8 +158,12 @@ struct ExternalScratch {
 };
 constexpr int kExternalCtlBytes = 8 * 4;
 constexpr int kExternalStatsBytes = 14 * 8;
-// Number of task ids of the factorization DAG (size of cnt / qhi / qlo).
+// Number of task ids of the FP64 factorization DAG (size of cnt / qhi / qlo).
 size_t factor_task_ids(const Geometry& g);
+// The fixed scratch of hqr_geqrf_noalloc, and what it carves for n_ids task
+// ids: T factors, counters, two queues, control words, statistics.
+constexpr size_t kNoAllocScratchBytes = size_t(64) << 20;
+size_t external_bytes(const Geometry& g, size_t n_ids);
 // Enqueue the factorization DAG on caller-supplied scratch.
 int launch_factor_external(const Geometry& g, const ExternalScratch& x, double* dA, double* dTAU,
                            long long timeout_ns, cudaStream_t stream);

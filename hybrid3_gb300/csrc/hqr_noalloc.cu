@@ -31,12 +31,11 @@
 
 namespace {
 
-constexpr size_t kNoAllocScratchBytes = size_t(64) << 20;
 constexpr int kMaxDevices = 64;
 
 // The scratch.  In host code this name only stands for the symbol; it is not
 // a device address.  The address comes from cudaGetSymbolAddress below.
-static __device__ __align__(256) unsigned char g_noalloc_scratch[kNoAllocScratchBytes];
+static __device__ __align__(256) unsigned char g_noalloc_scratch[hqr::kNoAllocScratchBytes];
 
 std::mutex g_noalloc_mu;
 void* g_noalloc_addr[kMaxDevices] = {};
@@ -77,12 +76,12 @@ extern "C" int hqr_geqrf_noalloc(long M, long N, int NB, int IB, double* dA, dou
   const size_t b_ids = round256(n_ids * sizeof(int));
   const size_t b_ctl = round256(hqr::kExternalCtlBytes);
   const size_t b_stats = round256(hqr::kExternalStatsBytes);
-  const size_t need = b_t + 3 * b_ids + b_ctl + b_stats;
-  if (need > kNoAllocScratchBytes) {
+  const size_t need = hqr::external_bytes(g, n_ids);
+  if (need > hqr::kNoAllocScratchBytes) {
     fprintf(stderr,
             "hqr_geqrf_noalloc: a %ld x %ld matrix with NB = %d needs %zu bytes of scratch; "
             "the fixed scratch holds %zu bytes\n",
-            M, N, NB, need, kNoAllocScratchBytes);
+            M, N, NB, need, hqr::kNoAllocScratchBytes);
     return HQR_ERR_UNSUPPORTED;
   }
   unsigned char* base = nullptr;

@@ -868,25 +868,13 @@ __device__ __noinline__ void panel_qr_general(double* R, int ldr, double* A, int
   __syncthreads();
 }
 
-// Points in a panel block where the DAG may act (see the executor's
-// PanelPhases): after the block's reflectors are stored, before its trailing
-// update, after the trailing update's first column block (first_cols wide)
-// and after the whole trailing update.  These do nothing.
-struct NoPanelPhases {
-  __device__ int first_cols(int cb, int) const { return cb; }
-  __device__ void after_panel() const {}
-  __device__ void before_trailing() const {}
-  __device__ void after_first() const {}
-  __device__ void after_trailing() const {}
-};
-
 // Inner block b of CORE_dgeqrt(NB, NB, IB, A, NB, T, NB, TAU): the QR of
 // columns [b w, (b+1) w) from row b w down (blocks 0..b-1 done), its T block,
-// and its application to the columns right of it.  It writes rows >= b w of
-// the tile only: rows [b w, (b+1) w) of R are final afterwards.
-template <typename RT = double, class Phases = NoPanelPhases>
+// and (trailing) its application to the columns right of it.  It writes rows
+// >= b w of the tile only: rows [b w, (b+1) w) of R are final afterwards.
+template <typename RT = double>
 __device__ void task_geqrt_blk(double* A, double* T, double* tau_g, const TileShape& sh, double* smem,
-                               const SmemPlan& sp, int b, const Phases& ph = Phases()) {
+                               const SmemPlan& sp, int b, bool trailing = true) {
   const int NB = sh.NB, w = sh.w;
   constexpr bool kFp64 = sizeof(RT) == sizeof(double);
   RT* sm = reinterpret_cast<RT*>(smem);
@@ -935,10 +923,8 @@ __device__ void task_geqrt_blk(double* A, double* T, double* tau_g, const TileSh
     store_block(T + i0 + (size_t)i0 * NB, NB, sTb, w, w, w);
     for (int e = threadIdx.x; e < w; e += kThreads) stg_cg(tau_g + i0 + e, double(sTau[e]));
     __syncthreads();
-    ph.after_panel();
-    ph.before_trailing();
-    for (int c0 = i0 + w, nc = ph.first_cols(sh.CB, w), first = 1; c0 < NB; c0 += nc, nc = sh.CB) {
-      const int ncol = min(nc, NB - c0);
+    for (int c0 = trailing ? i0 + w : NB; c0 < NB; c0 += sh.CB) {
+      const int ncol = min(sh.CB, NB - c0);
       RT* sC = sm + sp.off_c1;
       __syncthreads();
       load_block(sC, NB, A + i0 + (size_t)c0 * NB, NB, m, ncol);
@@ -946,12 +932,7 @@ __device__ void task_geqrt_blk(double* A, double* T, double* tau_g, const TileSh
       apply_block_t(A + i0 + (size_t)i0 * NB, NB, w, T + i0 + (size_t)i0 * NB, NB, w, m - w, true,
                     sC, NB, sC + w, NB, ncol, sm, sp, sh.RC, false, -1, resident);
       store_block(A + i0 + (size_t)c0 * NB, NB, sC, NB, m, ncol);
-      if (first) {
-        first = 0;
-        ph.after_first();
-      }
     }
-    ph.after_trailing();
   }
   __syncthreads();
 }
@@ -968,10 +949,10 @@ __device__ void task_geqrt_blk(double* A, double* T, double* tau_g, const TileSh
 // and is neither read nor written).  The reflectors keep A2's shape, so the
 // same arithmetic on A2 with zeros below the diagonal is exact, and only the
 // upper triangle is stored back.
-template <typename RT = double, class Phases = NoPanelPhases>
+template <typename RT = double>
 __device__ void task_tsqrt_blk(double* A1, double* A2, double* T, double* tau_g, const TileShape& sh,
                                double* smem, const SmemPlan& sp, int b, bool a2_upper = false,
-                               const Phases& ph = Phases()) {
+                               bool trailing = true) {
   const int NB = sh.NB, w = sh.w;
   constexpr bool kFp64 = sizeof(RT) == sizeof(double);
   RT* sm = reinterpret_cast<RT*>(smem);
@@ -1029,10 +1010,8 @@ __device__ void task_tsqrt_blk(double* A1, double* A2, double* T, double* tau_g,
     store_block(T + i0 + (size_t)i0 * NB, NB, sTb, w, w, w);
     for (int e = threadIdx.x; e < w; e += kThreads) stg_cg(tau_g + i0 + e, double(sTau[e]));
     __syncthreads();
-    ph.after_panel();
-    ph.before_trailing();
-    for (int c0 = i0 + w, nc = ph.first_cols(sh.CB, w), first = 1; c0 < NB; c0 += nc, nc = sh.CB) {
-      const int ncol = min(nc, NB - c0);
+    for (int c0 = trailing ? i0 + w : NB; c0 < NB; c0 += sh.CB) {
+      const int ncol = min(sh.CB, NB - c0);
       RT* sCt = sm + sp.off_c1;  // w x ncol rows of R (the panel area is free now)
       RT* sCb = sm + sp.off_c1 + w * sh.CB;  // NB x ncol of A2 after the R rows
       __syncthreads();
@@ -1047,12 +1026,36 @@ __device__ void task_tsqrt_blk(double* A1, double* A2, double* T, double* tau_g,
                     sCb, NB, ncol, sm, sp, sh.RC, false, a2_upper ? i0 : -1, resident);
       store_block(A1 + i0 + (size_t)c0 * NB, NB, sCt, w, w, ncol);
       store_block(A2 + (size_t)c0 * NB, NB, sCb, NB, mrows, ncol);
-      if (first) {
-        first = 0;
-        ph.after_first();
-      }
     }
-    ph.after_trailing();
+  }
+  __syncthreads();
+}
+
+// Columns [j w, (j+1) w) of the trailing update of inner block b of a panel
+// tile, as a task of its own: of a GEQRT (A2 null: V and C in the tile A1, on
+// rows >= b w) or of a TSQRT (rows [b w, (b+1) w) of R in A1, all of A2).
+template <typename RT = double>
+__device__ void task_trailing(double* A1, double* A2, const double* T, const TileShape& sh, double* smem,
+                              const SmemPlan& sp, int b, int j) {
+  const int NB = sh.NB, w = sh.w;
+  RT* sm = reinterpret_cast<RT*>(smem);
+  const int i0 = b * w;
+  const int m = A2 ? NB : NB - i0;
+  const double* V = A2 ? A2 + (size_t)i0 * NB : A1 + i0 + (size_t)i0 * NB;
+  for (int c0 = j * w; c0 < (j + 1) * w; c0 += sh.CB) {
+    const int ncol = min(sh.CB, (j + 1) * w - c0);
+    RT* sCt = sm + sp.off_c1;                                // the w x ncol rows of R (GEQRT: with the rows below)
+    RT* sCb = A2 ? sCt + w * sh.CB : sCt + w;
+    const int ldt = A2 ? w : NB;
+    double* top = A1 + i0 + (size_t)c0 * NB;
+    __syncthreads();
+    load_block(sCt, ldt, top, NB, A2 ? w : m, ncol);
+    if (A2) load_block(sCb, NB, A2 + (size_t)c0 * NB, NB, m, ncol);
+    __syncthreads();
+    apply_block_t(V, NB, A2 ? 0 : w, T + i0 + (size_t)i0 * NB, NB, w, A2 ? m : m - w, !A2, sCt, ldt, sCb, NB, ncol,
+                  sm, sp, sh.RC);
+    store_block(top, NB, sCt, ldt, A2 ? w : m, ncol);
+    if (A2) store_block(A2 + (size_t)c0 * NB, NB, sCb, NB, m, ncol);
   }
   __syncthreads();
 }
