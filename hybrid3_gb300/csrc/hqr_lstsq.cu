@@ -7,6 +7,7 @@
 // this is the first extension its callers need: x = R^-1 (Q^T b)(1:n), then
 // FP64 iterative refinement x += R^-1 (Q^T (b - A x))(1:n).
 #include "hqr_internal.h"
+#include "hqr_tile_fp64.cuh"
 
 namespace hqr {
 namespace {
@@ -177,7 +178,7 @@ __global__ void k_col_norm2(const double* __restrict__ R, long M, long ldr, doub
   }
 }
 
-// The two triangular solves give each block ONE right-hand side: FP64 issues
+// The triangular solves give each block ONE right-hand side: FP64 issues
 // at about one warp instruction per 70 cycles per SM sub-partition on this
 // part, so a block that carried several columns through the serial diagonal
 // solve spent most of each step there; one column per block spreads a step
@@ -296,6 +297,112 @@ __global__ void k_trsmt_step(const double* __restrict__ RA, int MT, int NB, doub
   Ck[r] = v;
 }
 
+// One step of a triangular solve over the first NT tile rows of C, tile orders
+// that are multiples of 32 up to kTriMaxNB, whose blocks find room for the
+// registers of a 32-column block (the others: k_trsm_step, k_trsmt_step): the same
+// steps and blocks, R Y = C from the bottom (TRANS false: step i updates the
+// blocks above i with Y_i, then solves block i - 1; i = NT solves only) or R^T
+// Y = C from the top (TRANS: step i updates the blocks from i on with Y_(i-1),
+// then solves block i).  Block (., q): one right-hand side, thread r = row r.
+//
+// A step is a chain (the next block's update, 4 us on one SM's FP64 pipe, then
+// its diagonal solve), so the solve is cut by 32 rows: warp b holds its rows'
+// 32 x 32 diagonal block in registers, divided by the diagonal (one shuffle and
+// one FMA a row instead of a barrier, a product and an FMA), and the blocks
+// beside it are loaded while the warp before it solves.  N = 8192, 16
+// right-hand sides: 64 steps of 27 us, 87 us before.
+constexpr int kTriMaxNB = 256;
+template <bool TRANS>
+__global__ void __launch_bounds__(kTriMaxNB) k_tri_step(const double* __restrict__ RA, int MT, int NB, double* __restrict__ C, int i, int NT) {
+  extern __shared__ double sm[];   // NB values of the solved block, NB of this one
+  double* sy = sm + NB;
+  const bool first = TRANS ? i == 0 : i == NT;   // nothing to update with yet
+  const int k = TRANS ? i + (int)blockIdx.x : (first ? NT - 1 : (int)blockIdx.x);
+  const int src = TRANS ? i - 1 : i;
+  const int q = blockIdx.y, tj = q / NB, cw = q % NB;
+  const int r = threadIdx.x, lane = r & 31, b = r >> 5, nb = NB >> 5;
+  const unsigned full = 0xffffffffu;
+  const long tile = (long)NB * NB;
+  double* Ck = C + ((long)k + (long)tj * MT) * tile + (long)cw * NB;
+  const bool diag = k == (TRANS ? i : (first ? NT - 1 : i - 1));
+  const double* Rkk = RA + ((long)k + (long)k * MT) * tile;
+  // element (r, 32 bb + j) of the triangular factor
+  auto at = [&](int bb, int j) { return TRANS ? Rkk[32 * bb + j + (long)r * NB] : Rkk[r + (long)(32 * bb + j) * NB]; };
+  double rs[32], inv = 0.0;
+  if (diag) {
+    inv = 1.0 / Rkk[r + (long)r * NB];
+#pragma unroll
+    for (int j = 0; j < 32; j++) rs[j] = (TRANS ? j < lane : j > lane) ? at(b, j) : 0.0;
+#pragma unroll
+    for (int j = 0; j < 32; j++) rs[j] *= __shfl_sync(full, inv, j);
+  }
+  double v = Ck[r];
+  if (!first) {
+    sm[r] = C[((long)src + (long)tj * MT) * tile + (long)cw * NB + r];
+    __syncthreads();
+    const double* Rt = TRANS ? RA + ((long)src + (long)k * MT) * tile : RA + ((long)k + (long)src * MT) * tile;
+    if (!TRANS) {
+      double a0 = 0.0, a1 = 0.0, a2 = 0.0, a3 = 0.0;
+#pragma unroll 4
+      for (int kk = 0; kk < NB; kk += 4) {
+        a0 = fma(Rt[r + (long)kk * NB], sm[kk], a0);
+        a1 = fma(Rt[r + (long)(kk + 1) * NB], sm[kk + 1], a1);
+        a2 = fma(Rt[r + (long)(kk + 2) * NB], sm[kk + 2], a2);
+        a3 = fma(Rt[r + (long)(kk + 3) * NB], sm[kk + 3], a3);
+      }
+      v -= (a0 + a1) + (a2 + a3);
+    } else {
+      // row r of R^T is a column of the tile: a warp takes its 32 rows four at
+      // a time, lanes down the columns
+      double dot = 0.0;
+#pragma unroll 1
+      for (int p = 0; p < 32; p += 4) {
+        double a[4] = {0.0, 0.0, 0.0, 0.0};
+        for (int kk = lane; kk < NB; kk += 32) {
+          const double y = sm[kk];
+#pragma unroll
+          for (int c = 0; c < 4; c++) a[c] = fma(Rt[kk + (long)(32 * b + p + c) * NB], y, a[c]);
+        }
+        warp_sums_fixed(a);
+#pragma unroll
+        for (int c = 0; c < 4; c++) dot = lane == p + c ? a[c] : dot;
+      }
+      v -= dot;
+    }
+  }
+  if (!diag) {
+    Ck[r] = v;
+    return;
+  }
+  for (int s = 0; s < nb; s++) {
+    const int bb = TRANS ? s : nb - 1 - s;
+    const bool later = TRANS ? b > bb : b < bb;
+    double pf[32];
+    if (later) {
+#pragma unroll
+      for (int j = 0; j < 32; j++) pf[j] = at(bb, j);
+    }
+    if (b == bb) {
+#pragma unroll
+      for (int jj = 0; jj < 32; jj++) {
+        const int j = TRANS ? jj : 31 - jj;
+        const double y = __shfl_sync(full, v, j);
+        if (TRANS ? lane > j : lane < j) v = fma(-rs[j], y, v);
+      }
+      v *= inv;
+      sy[r] = v;
+    }
+    __syncthreads();
+    if (later) {
+      double a[4] = {0.0, 0.0, 0.0, 0.0};
+#pragma unroll
+      for (int j = 0; j < 32; j++) a[j & 3] = fma(pf[j], sy[32 * bb + j], a[j & 3]);
+      v -= (a[0] + a[1]) + (a[2] + a[3]);
+    }
+  }
+  Ck[r] = v;
+}
+
 int blocks_for(long n) {
   long b = (n + 255) / 256;
   return (int)(b < 1 ? 1 : (b > 4 * 152 ? 4 * 152 : b));
@@ -375,6 +482,13 @@ size_t trsm_smem_bytes(int NB) { return ((size_t)NB * kRBlock + 2) * sizeof(doub
 
 int trsm_tiles(const double* dRA, long M, long N, int NB, double* dC, int nrhs, cudaStream_t s) {
   const int MT = (int)(M / NB), NT = (int)(N / NB);
+  if (NB % 32 == 0 && NB <= kTriMaxNB) {
+    for (int i = NT; i >= 1; i--)
+      k_tri_step<false><<<dim3((unsigned)(i < NT ? i : 1), (unsigned)nrhs), NB, 2 * NB * sizeof(double), s>>>(
+          dRA, MT, NB, dC, i, NT);
+    const cudaError_t e = cudaGetLastError();
+    return e == cudaSuccess ? HQR_OK : record_cuda_error(e, "k_tri_step launch");
+  }
   const size_t smem = trsm_smem_bytes(NB);
   if (smem > 48 * 1024) {
     cudaError_t e = cudaFuncSetAttribute(k_trsm_step, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
@@ -390,6 +504,13 @@ int trsm_tiles(const double* dRA, long M, long N, int NB, double* dC, int nrhs, 
 
 int trsmt_tiles(const double* dRA, long M, long N, int NB, double* dC, int nrhs, cudaStream_t s) {
   const int MT = (int)(M / NB), NT = (int)(N / NB);
+  if (NB % 32 == 0 && NB <= kTriMaxNB) {
+    for (int i = 0; i < NT; i++)
+      k_tri_step<true><<<dim3((unsigned)(NT - i), (unsigned)nrhs), NB, 2 * NB * sizeof(double), s>>>(dRA, MT, NB, dC,
+                                                                                                     i, NT);
+    const cudaError_t e = cudaGetLastError();
+    return e == cudaSuccess ? HQR_OK : record_cuda_error(e, "k_tri_step launch");
+  }
   const size_t smem = trsm_smem_bytes(NB);
   if (smem > 48 * 1024) {
     cudaError_t e = cudaFuncSetAttribute(k_trsmt_step, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
