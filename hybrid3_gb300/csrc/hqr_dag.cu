@@ -9,10 +9,11 @@
 
 namespace hqr {
 
-// Task ids of the plain FP64 factorization without trailing-update tasks, and
-// the bytes of scratch that hqr_geqrf_noalloc carves for n_ids ids.
-static size_t coarse_task_ids(const Geometry& g) {
-  return (size_t)g.steps * g.MT * (g.NB / g.w) + (size_t)g.steps * g.NT * g.MT * g.NC;
+// Task ids of the plain FP64 factorization with nc column blocks per update
+// tile and no trailing-update tasks, and the bytes of scratch that
+// hqr_geqrf_noalloc carves for n_ids ids.
+static size_t coarse_task_ids(const Geometry& g, int nc) {
+  return (size_t)g.steps * g.MT * (g.NB / g.w) + (size_t)g.steps * g.NT * g.MT * nc;
 }
 size_t external_bytes(const Geometry& g, size_t n_ids) {
   auto round256 = [](size_t b) { return (b + 255) & ~size_t(255); };
@@ -153,7 +154,6 @@ static int launch_exec(const DagParams& p, const Geometry& g, cudaStream_t strea
 }
 
 static int run_dag(DagParams& p, DagWorkspace* ws, const Geometry& g, cudaStream_t stream) {
-  p.sh = shape_of(g);
   p.sp = SmemPlan::make(p.sh);
   p.n_ids = id_end(p);
   int rc = dag_workspace_reserve(ws, (size_t)p.n_ids);
@@ -197,12 +197,62 @@ static FineSteps fine_steps(const Geometry& g, bool split) {
   if (nblk < 2) return f;
   f.ids = (long long)(g.steps - f.from) * g.MT * nblk * nblk;
   for (int i = f.from; i < g.steps; i++) f.tasks += (g.MT - i) * nblk * (nblk - 1) / 2;
-  // the allocation-free entry point has the same tasks, hence the same
-  // rounding: where its scratch holds the factorization without these ids but
-  // not with them, neither has them
-  const size_t plain = external_bytes(g, coarse_task_ids(g));
-  const bool squeezed = plain <= kNoAllocScratchBytes && external_bytes(g, coarse_task_ids(g) + f.ids) > kNoAllocScratchBytes;
-  if ((!split && squeezed) || (long long)coarse_task_ids(g) + f.ids > 0x3fffffffLL) f.ids = f.tasks = 0;
+  if ((long long)coarse_task_ids(g, split ? 2 : g.NC) + f.ids > 0x3fffffffLL) f.ids = f.tasks = 0;
+  return f;
+}
+
+// Columns per FP64 update task: the tile's nominal block (g.CB), or fewer
+// where the longest chain of updates (`path` tasks) sets the pace rather than
+// all `tiles` of them (`cols` columns of data each) on every SM.  A task of cb
+// columns takes cb + c0 column times, c0 about 4, 14 at tile order 64
+// (measured, us, CB 64 / 32 / 16 / 8: NB 64 183 / 100 / 63 / 49; NB 128 635 /
+// 337 / 180 / 108; NB 256 - / 1251 / 674 / 414).
+static int update_columns(const Geometry& g, long long tiles, long long path, int cols) {
+  const double c0 = std::max(4.0, 57344.0 / ((double)g.NB * g.NB));
+  int best = g.CB;
+  double t_best = 0.0;
+  for (int cb = g.CB; cb >= 8; cb -= 8) {
+    const long long tasks = tiles * ((cols + cb - 1) / cb);
+    if (g.CB % cb != 0 || tasks > 0x0fffffffLL) continue;
+    const double t = (cb + c0) * std::max((double)path, (double)tasks / dag_sm_count());
+    if (cb == g.CB || t < 0.95 * t_best) {
+      best = cb;
+      t_best = t;
+    }
+  }
+  return best;
+}
+static void set_columns(DagParams& p, const Geometry& g, int cb, int cols) {
+  p.sh = shape_of(g);
+  if (p.oz) return;
+  p.sh.CB = cb;
+  p.NC = (cols + cb - 1) / cb;
+  p.count_every = g.CB / cb;
+}
+// The same for C <- Q^T C or Q C on CT tile columns (ccols > 0: that many
+// columns hold data; in a single tile column only their blocks are tasks).
+static void set_apply_columns(DagParams& p, const Geometry& g, long long tiles, long long path, int CT,
+                              long long ccols) {
+  const int cols = CT == 1 && ccols > 0 && ccols < g.NB ? (int)ccols : g.NB;
+  set_columns(p, g, update_columns(g, tiles, path, cols), cols);
+}
+
+// The FP64 factorization's update columns and fine steps.  The allocation-free
+// entry point runs the same tasks, hence with the same rounding: where its
+// scratch holds the plain tasks' ids but not these, both take the plain ones.
+struct FactorTasks {
+  int cb;
+  FineSteps fine;
+  size_t ids;
+};
+static FactorTasks factor_tasks(const Geometry& g) {
+  long long tiles = 0;
+  for (int i = 0; i < g.steps; i++) tiles += (long long)(g.NT - 1 - i) * (g.MT - i);
+  FactorTasks f{update_columns(g, tiles, g.MT + g.steps, g.NB), fine_steps(g, false), 0};
+  f.ids = coarse_task_ids(g, g.NB / f.cb) + (size_t)f.fine.ids;
+  if (external_bytes(g, coarse_task_ids(g, g.NC)) <= kNoAllocScratchBytes &&
+      external_bytes(g, f.ids) > kNoAllocScratchBytes)
+    f = FactorTasks{g.CB, FineSteps{}, coarse_task_ids(g, g.NC)};
   return f;
 }
 
@@ -269,7 +319,15 @@ int launch_factor(const Geometry& g, DagWorkspace* ws, double* dA, double* dT, d
   p.prep = p.oz;
   p.nblk = g.NB / g.w;
   set_tree(p, g, tw);
-  const FineSteps fine = p.tree == 0 ? fine_steps(g, p.oz != 0) : FineSteps{};
+  FineSteps fine;
+  int cb = g.CB;
+  if (p.tree == 0 && p.oz) fine = fine_steps(g, true);
+  if (p.tree == 0 && !p.oz) {
+    const FactorTasks f = factor_tasks(g);
+    fine = f.fine;
+    cb = f.cb;
+  }
+  set_columns(p, g, cb, g.NB);
   p.fine_from = fine.from;
   p.fine_ids = (int)fine.ids;
   // tasks: per step i, nblk inner blocks of each of the MT-i panel tiles [+ one
@@ -306,6 +364,7 @@ int launch_apply_qt(const Geometry& g, DagWorkspace* ws, const double* dA, doubl
   long long tiles = 0;
   for (int i = 0; i < g.steps; i++) tiles += (long long)CT * (g.MT - i);
   set_oz(p, g, ozw, oz_chunks(tiles, g.MT + g.steps, ccols));
+  set_apply_columns(p, g, tiles, g.MT + g.steps, CT, ccols);
   p.prep = 0;
   p.nblk = 1;
   // rebuild_t: panel tasks rebuild each panel tile's T (FP64: its diagonal
@@ -337,6 +396,7 @@ int launch_apply_qt_tree(const Geometry& g, DagWorkspace* ws, const double* dA, 
   long long tiles = 0;
   for (int i = 0; i < g.steps; i++) tiles += (long long)CT * (g.MT - i);
   set_oz(p, g, ozw, oz_chunks(tiles, tw->S + (g.MT + tw->S - 1) / tw->S + g.steps));
+  set_apply_columns(p, g, tiles, tw->S + (g.MT + tw->S - 1) / tw->S + g.steps, CT, 0);
   p.prep = 0;
   p.nblk = 1;
   p.skip_panels = 1;   // the T factors / slices of the factorization on this plan
@@ -365,6 +425,7 @@ int launch_build_q(const Geometry& g, DagWorkspace* ws, const double* dA, double
   long long tiles = 0;
   for (int i = 0; i < g.steps; i++) tiles += (long long)(g.NT - i) * (g.MT - i);
   set_oz(p, g, ozw, oz_chunks(tiles, g.MT + g.steps));
+  set_columns(p, g, update_columns(g, tiles, g.MT + g.steps, g.NB), g.NB);
   p.prep = 0;
   p.nblk = 1;
   p.skip_panels = rebuild_t ? 0 : 1;   // as in launch_apply_qt (split: T from its own slot)
@@ -396,6 +457,7 @@ int launch_apply_q(const Geometry& g, DagWorkspace* ws, const double* dA, double
   long long tiles = 0;
   for (int i = 0; i < g.steps; i++) tiles += (long long)CT * (g.MT - i);
   set_oz(p, g, ozw, oz_chunks(tiles, g.MT + g.steps, ccols));
+  set_apply_columns(p, g, tiles, g.MT + g.steps, CT, ccols);
   p.prep = 0;
   p.nblk = 1;
   p.skip_panels = rebuild_t ? 0 : 1;
@@ -571,7 +633,7 @@ size_t tree_slots(const Geometry& g, int S) {
   return (size_t)g.steps * ((g.MT + S - 1) / S);
 }
 
-size_t factor_task_ids(const Geometry& g) { return coarse_task_ids(g) + (size_t)fine_steps(g, false).ids; }
+size_t factor_task_ids(const Geometry& g) { return factor_tasks(g).ids; }
 
 int launch_factor_external(const Geometry& g, const ExternalScratch& x, double* dA, double* dTAU,
                            long long timeout_ns, cudaStream_t stream) {
@@ -582,19 +644,19 @@ int launch_factor_external(const Geometry& g, const ExternalScratch& x, double* 
   p.MT = g.MT;
   p.NT = g.NT;
   p.CT = g.NT;
-  p.NC = g.NC;
   p.steps = g.steps;
   p.J = g.NT;
   p.nblk = g.NB / g.w;
-  p.sh = shape_of(g);
+  const FactorTasks f = factor_tasks(g);
+  const FineSteps& fine = f.fine;
+  set_columns(p, g, f.cb, g.NB);
   p.sp = SmemPlan::make(p.sh);
-  const FineSteps fine = fine_steps(g, false);
   p.fine_from = fine.from;
   p.fine_ids = (int)fine.ids;
-  p.n_ids = (int)factor_task_ids(g);
+  p.n_ids = (int)f.ids;
   long long n = fine.tasks;
   for (int i = 0; i < g.steps; i++)
-    n += (long long)(g.MT - i) * p.nblk + (long long)g.NC * (g.NT - 1 - i) * (g.MT - i);
+    n += (long long)(g.MT - i) * p.nblk + (long long)p.NC * (g.NT - 1 - i) * (g.MT - i);
   p.n_tasks = (int)n;
   p.A = dA;
   p.T = x.T;

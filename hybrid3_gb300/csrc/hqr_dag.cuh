@@ -87,6 +87,9 @@ struct DagParams {
   int mode;
   int MT, NT, CT, NC, steps, J;   // J = tile columns spanned by update ids
   int nblk;                        // panel inner blocks per panel task id (factorization: NB / w)
+  // update tasks that are narrower than the tile's nominal column block: one
+  // in count_every is counted in the statistics (0, 1: all)
+  int count_every;
   // Domain tree (tree > 0): at step i the tile rows i.. are cut into domains of
   // `tree` tiles; each domain runs the flat TS chain on its own top tile, then
   // the domain tops' R are merged into R(i, i) one after the other by TT
@@ -866,7 +869,8 @@ __global__ void __launch_bounds__(kThreads, BATCH ? 2 : 1) dag_exec_kernel(DagPa
     __syncthreads();
     if (threadIdx.x == 0) {
       const int slot = t.type == kTRAIL ? (t.k > t.i ? kTSQRT : kGEQRT) : stat_slot(t.type);
-      const int counted = t.type == kTRAIL ? 0 : 1;   // (GEQRT / TSQRT: one per panel block)
+      const bool update = t.type == kLARFB || t.type == kSSRFB || t.type == kTTMQR;
+      const int counted = t.type == kTRAIL || (update && q.count_every > 1 && t.c % q.count_every != 0) ? 0 : 1;
       local_cnt[slot] += counted;
       const long long c1 = clock64();
       local_cyc[slot] += (unsigned long long)(c1 - c0);
