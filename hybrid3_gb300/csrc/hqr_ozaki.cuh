@@ -72,7 +72,7 @@ constexpr int kBStages = 4;
 // done barriers: one per chunk in flight on either ring, so that no two
 // chunks a wait may still refer to share a barrier (parity waits stay exact)
 constexpr int kDoneStages = kAStages > kBStages ? kAStages : kBStages;
-constexpr int kSlicerWarps = kWarps - 1;   // warp 0 issues the copies and the MMAs
+constexpr int kSlicerWarps = kWarps - 2;   // warp 0 issues the MMAs, warp 1 the copies of A
 // Barriers: a_full[kAStages] (TMA bytes), b_full[kBStages] (one arrival per
 // slicer warp), done[kDoneStages] (tcgen05.commit of one chunk's MMAs).
 constexpr int kBarAFull = 0, kBarBFull = kAStages, kBarDone = kAStages + kBStages;
@@ -105,18 +105,22 @@ __device__ __forceinline__ void mbar_expect_tx(uint64_t* b, uint32_t bytes) {
 // Wait for the phase with parity `parity`, bounded by kWaitNs of wall time
 // and abandoned at once when the scheduler's error word is set; false then.
 constexpr long long kWaitNs = 2000000000LL;
+__device__ __forceinline__ bool mbar_try(uint32_t a, uint32_t parity) {
+  uint32_t done;
+  asm volatile(
+      "{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+      "selp.u32 %0, 1, 0, p;\n\t}"
+      : "=r"(done)
+      : "r"(a), "r"(parity)
+      : "memory");
+  return done != 0;
+}
 __device__ __forceinline__ bool mbar_wait(uint64_t* b, uint32_t parity, const unsigned* err) {
   const uint32_t a = smem_u32(b);
+  if (mbar_try(a, parity)) return true;
   const uint64_t t0 = global_ns();
   for (long long it = 0; it < kWaitIters; it++) {
-    uint32_t done;
-    asm volatile(
-        "{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
-        "selp.u32 %0, 1, 0, p;\n\t}"
-        : "=r"(done)
-        : "r"(a), "r"(parity)
-        : "memory");
-    if (done) return true;
+    if (mbar_try(a, parity)) return true;
     if ((it & 255) == 255) {
       if (*((volatile const unsigned*)err) != 0u) return false;
       if ((long long)(global_ns() - t0) > kWaitNs) return false;
@@ -317,7 +321,7 @@ struct Ctx {
   double* sY;           // the right operand: kK x kN doubles, ld kLdY
   uint32_t tmem;        // base of the 512 TMEM columns
   int n;                // K chunks consumed so far in this task (same in every thread)
-  int na;               // K chunks whose A copy has been issued (warp 0 only)
+  int na;               // K chunks whose A copy has been issued (warp 1 only)
   int yb;               // which half of sEb describes sY
   unsigned* err;        // scheduler error word
 };
@@ -493,20 +497,20 @@ __device__ __forceinline__ bool wait_chunk(const Ctx& c, int base, int stages, i
   return mbar_wait(c.bar + base + n % stages, (uint32_t)((n / stages) & 1), c.err);
 }
 // Chunk `chunk` of X into A stage n: its digit planes 0..G-1 (the first G x 4
-// KiB of the chunk).  Warp 0, one lane of which issues the copy.
+// KiB of the chunk).  Warp 1, one lane of which issues the copy.
 template <int G = kGroups>
 __device__ __forceinline__ void issue_a(Ctx& c, const uint8_t* X, int chunk, int n) {
-  if (threadIdx.x != 0) return;
+  if (threadIdx.x != 32) return;
   uint64_t* b = c.bar + kBarAFull + n % kAStages;
   mbar_expect_tx(b, G * kSliceABytes);
   tma_load_1d(c.sA + (n % kAStages) * kAChunkBytes, X + (size_t)chunk * kAChunkBytes, G * kSliceABytes, b);
 }
 
 // Issue the bulk copies of the first chunks of the next product's left
-// operand X (warp 0), e.g. before the right operand is staged.
+// operand X (warp 1), e.g. before the right operand is staged.
 template <int G = kGroups>
 __device__ __forceinline__ void prefetch(Ctx& c, const uint8_t* X) {
-  if (threadIdx.x < 32) {
+  if ((threadIdx.x >> 5) == 1) {
     fence_proxy_async_global();
     for (; c.na < c.n + kAStages; c.na++) issue_a<G>(c, X, c.na - c.n, c.na);
   }
@@ -519,10 +523,13 @@ __device__ __forceinline__ void slicer_sync() {
 
 // The 8 t-group accumulators of X (prepared slices) times the staged right
 // operand; Xnext (or nullptr): the left operand of the next product, whose
-// first chunks are fetched as soon as their stages are free.  Warp 0 (one
-// elected lane): bulk copies of A and the MMAs; warps 1..7: slicing of B, up to
-// kBStages chunks ahead of the MMAs.  On return (true) the accumulators are
-// final in TMEM.  G < 8: only the pairs of weight p + q < G (accumulators
+// first chunks are fetched as soon as their stages are free.  Warp 0: the
+// MMAs and nothing else, since the tensor core holds only a few of them in
+// advance and idles through whatever else the warp does between two chunks.
+// Warp 1: the bulk copies of A (about 330 cycles each with the look at the
+// stage: on warp 0 or on a slicer they held up every chunk).  Warps 2..7:
+// slicing of B, up to kBStages chunks ahead of the MMAs.  On return (true) the
+// accumulators are final in TMEM.  G < 8: only the pairs of weight p + q < G (accumulators
 // 0..G-1; the others are left as they are).  nch: K chunks (8, or 16 for a
 // K = 256 product whose right operand's second half, `reload` (global, kK x
 // kN, ld kK), replaces the staged one once the slicers are past chunk 7; the
@@ -538,10 +545,7 @@ inline __device__ bool gemm(Ctx& c, const uint8_t* X, const uint8_t* Xnext, int 
     const uint32_t id = idesc_bf16(kM, kN);
     const uint64_t dA0 = sdesc(smem_u32(c.sA), 128, 256);
     const uint64_t dB0 = sdesc(smem_u32(c.sB), 128, 256);
-    fence_proxy_async_global();
-    // chunks of this product not prefetched yet (stages free: every earlier MMA is done)
-    for (; c.na < n0 + kAStages; c.na++) issue_a<G>(c, X, c.na - n0, c.na);
-    for (int j = 0; j < nch && ok; j++) {
+    for (int j = 0; j < nch; j++) {
       const int n = n0 + j;
       ok = wait_chunk(c, kBarAFull, kAStages, n) && wait_chunk(c, kBarBFull, kBStages, n);
       ok = __all_sync(0xffffffffu, ok);
@@ -555,11 +559,10 @@ inline __device__ bool gemm(Ctx& c, const uint8_t* X, const uint8_t* Xnext, int 
       for (int p = 0; p < kS && p < G; p++) {
 #pragma unroll
         for (int q = 0; q < kS && p + q < G; q++) {
-          const int first_p = (p + q) - (kS - 1) > 0 ? (p + q) - (kS - 1) : 0;
-          const uint32_t acc = (j > 0 || p > first_p) ? 1u : 0u;
+          const uint32_t acc = (j > 0 || p > 0) ? 1u : 0u;
           const uint32_t d = c.tmem + (uint32_t)((p + q) * kN);
           const uint64_t a = dA + (uint64_t)((p * kSliceABytes) >> 4), b = dB + (uint64_t)((q * kSliceBBytes) >> 4);
-          const int last_q = (G < kS ? G : kS) - 1 - p;   // slice p's last product
+          const int last_q = G - 1 - p;   // slice p's last product
           if (last_q == 0)
             mma_bf16<kARead>(d, a, b, id, acc);
           else if (q == 0)
@@ -571,29 +574,25 @@ inline __device__ bool gemm(Ctx& c, const uint8_t* X, const uint8_t* Xnext, int 
         }
       }
       mma_commit(c.bar + kBarDone + n % kDoneStages);
-      // refill the A stage of chunk n - 1 with chunk n - 1 + kAStages once its MMAs are done
-      if (j >= 1 && j + kAStages - 1 < nch) {
-        ok = __all_sync(0xffffffffu, wait_chunk(c, kBarDone, kDoneStages, n - 1));
-        if (!ok) break;
-        issue_a<G>(c, X, j + kAStages - 1, n + kAStages - 1);
-        c.na = n + kAStages;
-      }
-    }
-    // prefetch the next product's first chunks into the stages of the last kAStages
-    if (ok && Xnext) {
-      for (int j = 0; j < kAStages; j++) {
-        ok = __all_sync(0xffffffffu, wait_chunk(c, kBarDone, kDoneStages, n0 + nch - kAStages + j));
-        if (!ok) break;
-        issue_a<G>(c, Xnext, j, n0 + nch + j);
-      }
-      if (ok) c.na = n0 + nch + kAStages;
     }
     __syncwarp();
+  } else if (warp == 1) {
+    // X's chunks not prefetched yet, then the first kAStages of Xnext, each
+    // once the MMAs of the chunk that held its stage are done
+    fence_proxy_async_global();
+    for (const int end = n0 + nch + (Xnext ? kAStages : 0); c.na < end; c.na++) {
+      const int m = c.na - kAStages;
+      if (m >= n0) ok = __all_sync(0xffffffffu, wait_chunk(c, kBarDone, kDoneStages, m));
+      if (!ok) break;
+      const bool next = c.na >= n0 + nch;
+      issue_a<G>(c, next ? Xnext : X, c.na - n0 - (next ? nch : 0), c.na);
+      __syncwarp();
+    }
   } else {
-    // slicer thread ts owns quads ts, ts + 224, ... of the product's nch x 256;
+    // slicer thread ts owns quads ts, ts + 192, ... of the product's nch x 256;
     // every slicer thread passes every loop step and the reload barriers, so
     // a failed wait (ok false, warp-uniform) skips work but never a barrier
-    const int ts = threadIdx.x - 32;
+    const int ts = threadIdx.x - 64;
     constexpr int kStride = kSlicerWarps * 32;
     int g = ts;
     for (int j = 0; j < nch; j++) {
@@ -686,7 +685,6 @@ __device__ __forceinline__ double recombine(const uint32_t (&acc)[kGroups][kDC],
 // Epilogue modes (R = the product just computed).
 enum Epi : int {
   kEpiStore = 0,      // g = R                                   (global)
-  kEpiToY = 1,        // sY = gm + R (gm global, may be null)    -> next right operand
   kEpiToYSubTop = 2,  // sY = R; gm -= R (gm global, may be null) -> next right operand
   kEpiSubInto = 3,    // g -= R                                  (global)
 };
@@ -706,7 +704,7 @@ inline __device__ void drain(Ctx& c, const int* Ea, int mode, double* g, int ldg
   const int cb = kColsPerWarp * (w >> 2);
   const int ea = __ldcg(Ea + row);
   const uint32_t lane_addr = c.tmem + ((uint32_t)(32 * (w & 3)) << 16);
-  const bool to_y = (mode == kEpiToY || mode == kEpiToYSubTop);
+  const bool to_y = mode == kEpiToYSubTop;
   const int nb = c.yb ^ 1;   // exponents of the new right operand
   if (to_y) {
     if (threadIdx.x < kN) c.sEb[nb * kN + threadIdx.x] = 0;
@@ -727,28 +725,28 @@ inline __device__ void drain(Ctx& c, const int* Ea, int mode, double* g, int ldg
       tmem_ld_groups(lane_addr + (uint32_t)c0, acc);
     else
       tmem_ld_groups4(lane_addr + (uint32_t)c0, acc);
+    unsigned emax[kDC];
 #pragma unroll
     for (int i = 0; i < kDC; i++) {
       const int col = c0 + i;
       const int eb = c.sEb[c.yb * kN + col];
       const double r = recombine(acc, i, ea + eb - (kExpBias + 1023), ea > 0 && eb > 0);
       const size_t o = (size_t)col;
-      double y = 0.0;
       if (mode == kEpiStore) {
         stg_cg(g + row + o * ldg, r);
-      } else if (mode == kEpiToY) {
-        y = mem[i] + r;
-      } else if (mode == kEpiToYSubTop) {
-        y = r;
+      } else if (to_y) {
+        c.sY[col * kLdY + row] = r;
         if (gm) stg_cg(gm + row + o * ldm, mem[i] - r);
+        emax[i] = __reduce_max_sync(0xffffffffu, (unsigned)biased_exp(r));
       } else {
         stg_cg(g + row + o * ldg, mem[i] - r);
       }
-      if (to_y) {
-        c.sY[col * kLdY + row] = y;
-        const unsigned e = __reduce_max_sync(0xffffffffu, (unsigned)biased_exp(y));
-        if (lane == 0) atomicMax(c.sEb + nb * kN + col, (int)e);
-      }
+    }
+    if (to_y) {   // lane i: column c0 + i (an atomic per column from one lane cost 5 kcycles an epilogue)
+      unsigned e = emax[0];
+#pragma unroll
+      for (int i = 1; i < kDC; i++) e = lane == i ? emax[i] : e;
+      if (lane < kDC) atomicMax(c.sEb + nb * kN + c0 + lane, (int)e);
     }
   }
   tc_fence_before();
