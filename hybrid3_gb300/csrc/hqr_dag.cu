@@ -184,15 +184,17 @@ static int run_dag(DagParams& p, DagWorkspace* ws, const Geometry& g, cudaStream
 // the shorter chain gains.  Measured, against whole panel blocks: FP64 n =
 // 2048, NB 256: factorization 73 -> 38 ms; n = 4096: 155 -> 118 ms; split n =
 // 3072 (against blocks that released their dependents in phases): QR + Q 35.7
-// -> 28.4 ms; split n = 16384 unchanged.
+// -> 28.4 ms; split n = 16384 unchanged.  FP32 panels have no such steps: their
+// blocks take half the time and are latency, not work (32768 x 8192: 355 ms
+// with none, 356 from 300 tiles on, 382 from 6000).
 struct FineSteps {
   int from = 0;
   long long ids = 0, tasks = 0;
 };
-constexpr long long kFineTilesSplit = 6000, kFineTilesFp64 = 600;
-static FineSteps fine_steps(const Geometry& g, bool split) {
+constexpr long long kFineTilesSplit = 6000, kFineTilesFp64 = 600, kFineTilesFp32 = 0;
+static FineSteps fine_steps(const Geometry& g, bool split, bool fp32 = false) {
   FineSteps f;
-  const long long nblk = g.NB / g.w, tiles = split ? kFineTilesSplit : kFineTilesFp64;
+  const long long nblk = g.NB / g.w, tiles = fp32 ? kFineTilesFp32 : split ? kFineTilesSplit : kFineTilesFp64;
   while (f.from < g.steps && (long long)(g.NT - f.from - 1) * (g.MT - f.from - 1) > tiles) f.from++;
   if (nblk < 2) return f;
   f.ids = (long long)(g.steps - f.from) * g.MT * nblk * nblk;
@@ -321,7 +323,7 @@ int launch_factor(const Geometry& g, DagWorkspace* ws, double* dA, double* dT, d
   set_tree(p, g, tw);
   FineSteps fine;
   int cb = g.CB;
-  if (p.tree == 0 && p.oz) fine = fine_steps(g, true);
+  if (p.tree == 0 && p.oz) fine = fine_steps(g, true, p.oz_p32 != 0);
   if (p.tree == 0 && !p.oz) {
     const FactorTasks f = factor_tasks(g);
     fine = f.fine;
