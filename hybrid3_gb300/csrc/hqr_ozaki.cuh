@@ -12,7 +12,7 @@
 //     its largest element and written as a fixed-point integer F, |F| < 2^62,
 //     so an element 2^-9 of its row maximum still keeps 53 bits;
 //   * F is split into kS = 8 signed digits of kRho = 8 bits, |d_0| <= 64,
-//     |d_p| <= 128, F = sum_p d_p 2^(8 (7 - p)); every digit is an exact BF16
+//     |d_p| <= 128, F = sum_p d_p 2^(8 (7 - p)); every digit is an exact FP16
 //     value;
 //   * the slice products X_p Y_q with p + q <= 7 (0-based; 36 of the 64) are
 //     exact on the tensor cores: |d_x d_y| <= 2^14, a K = 128 sum stays below
@@ -32,7 +32,7 @@
 // memory (staged from HBM for the first product of an update, written there
 // by the previous product's epilogue otherwise) and is sliced chunk by chunk
 // into a double-buffered stage while the MMAs of the previous chunk run.
-// MMAs are issued by one thread (M = 128, N = 64, K = 16, BF16 x BF16 ->
+// MMAs are issued by one thread (M = 128, N = 64, K = 16, FP16 x FP16 ->
 // FP32).  Every mbarrier wait is bounded; on time-out the error word is set
 // and the task is abandoned.
 #pragma once
@@ -45,7 +45,7 @@ namespace oz {
 constexpr int kK = 128;            // the tile order: K (and M) of every product
 constexpr int kN = 64;             // columns of the right operand (MMA N)
 constexpr int kM = 128;            // rows per MMA (one TMEM lane per row)
-constexpr int kKC = 16;            // K per BF16 MMA
+constexpr int kKC = 16;            // K per FP16 MMA
 constexpr int kChunks = kK / kKC;  // 8 K chunks per product
 constexpr int kRho = 8;            // bits per digit
 constexpr int kS = 8;              // digits (slices) per element
@@ -171,10 +171,9 @@ __device__ __forceinline__ uint64_t sdesc(uint32_t addr, uint32_t lbo, uint32_t 
   return (uint64_t)((addr & 0x3FFFF) >> 4) | ((uint64_t)((lbo >> 4) & 0x3FFF) << 16) |
          ((uint64_t)((sbo >> 4) & 0x3FFF) << 32) | ((uint64_t)1 << 46);
 }
-// Instruction descriptor: kind::f16, BF16 x BF16 -> FP32, K-major A and B.
-__device__ __forceinline__ uint32_t idesc_bf16(int M, int N) {
-  return (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(N >> 3) << 17) |
-         ((uint32_t)(M >> 4) << 24);
+// Instruction descriptor: kind::f16, FP16 x FP16 -> FP32, K-major A and B.
+__device__ __forceinline__ uint32_t idesc_f16(int M, int N) {
+  return (1u << 4) | ((uint32_t)(N >> 3) << 17) | ((uint32_t)(M >> 4) << 24);
 }
 // MMAs and their commits are issued by one elected lane of a converged warp
 // (every lane executes the instruction, predicated): the operands then stay
@@ -186,22 +185,22 @@ __device__ __forceinline__ uint32_t idesc_bf16(int M, int N) {
 // without; 32 is the tensor work).
 enum ACollect : int { kARead = 0, kAFill = 1, kAUse = 2, kALast = 3 };
 template <int COLLECT>
-__device__ __forceinline__ void mma_bf16(uint32_t d_tmem, uint64_t a, uint64_t b, uint32_t id,
+__device__ __forceinline__ void mma_f16(uint32_t d_tmem, uint64_t a, uint64_t b, uint32_t id,
                                          uint32_t accumulate) {
-#define HQR_MMA_BF16(USE)                                                                  \
+#define HQR_MMA_F16(USE)                                                                  \
   asm volatile(                                                                            \
       "{\n\t.reg .pred p, l;\n\telect.sync _|l, 0xffffffff;\n\tsetp.ne.b32 p, %4, 0;\n\t"   \
       "@l tcgen05.mma.cta_group::1.kind::f16" USE " [%0], %1, %2, %3, p;\n\t}" ::"r"(d_tmem), \
       "l"(a), "l"(b), "r"(id), "r"(accumulate))
   if (COLLECT == kAFill)
-    HQR_MMA_BF16(".collector::a::fill");
+    HQR_MMA_F16(".collector::a::fill");
   else if (COLLECT == kAUse)
-    HQR_MMA_BF16(".collector::a::use");
+    HQR_MMA_F16(".collector::a::use");
   else if (COLLECT == kALast)
-    HQR_MMA_BF16(".collector::a::lastuse");
+    HQR_MMA_F16(".collector::a::lastuse");
   else
-    HQR_MMA_BF16("");
-#undef HQR_MMA_BF16
+    HQR_MMA_F16("");
+#undef HQR_MMA_F16
 }
 __device__ __forceinline__ void mma_commit(uint64_t* bar) {
   asm volatile(
@@ -283,26 +282,65 @@ __device__ __forceinline__ long long fixed_of(double x, int E) {
   const unsigned long long F = (k == 0) ? t : (((t >> (k - 1)) + 1ULL) >> 1);
   return (b < 0) ? -(long long)F : (long long)F;
 }
-// Balanced base-256 digits d_0..d_7 of F (|F| < 2^62) as exact floats:
-// F = sum d_p 2^(8 (7 - p)), d_1..d_7 in [-128, 127], d_0 in [-64, 64].
-// Adding 128 at each of the seven low byte positions, G = F + 0x80808080808080
-// (no overflow: |G| < 2^63), lets the carries do the balancing: byte j of G is
-// d_(7-j) + 128 (j < 7) and G >> 56 is d_0.  The float of byte b - 128 is
-// (2^23 + b) - (2^23 + 128), with 2^23 + b assembled by one byte permute:
-// exact, no conversion unit.
-__device__ __forceinline__ void digits(long long F, float* d) {
-  const long long G = F + 0x0080808080808080LL;
-  const uint32_t lo = (uint32_t)G, hi = (uint32_t)((unsigned long long)G >> 32);
-#pragma unroll
-  for (int j = 0; j < kS - 1; j++) {
-    const uint32_t bits = __byte_perm(j < 4 ? lo : hi, 0x4B000000u, 0x7440u | (uint32_t)(j & 3));
-    d[kS - 1 - j] = __uint_as_float(bits) - 8388736.0f;
-  }
-  d[0] = (float)(int)(G >> 56);
+// The balanced base-256 digits d_0..d_7 of F (|F| < 2^62), F = sum d_p 2^(8 (7
+// - p)), d_1..d_7 in [-128, 127], d_0 in [-64, 64]: with 128 added at every byte
+// position, G = F + 0x8080808080808080 (as unsigned 64-bit), the carries do
+// the balancing and byte 7 - p of G is d_p + 128.
+__device__ __forceinline__ void offset_digits_general(double x, int E, uint32_t& lo, uint32_t& hi) {
+  const unsigned long long G = (unsigned long long)fixed_of(x, E) + 0x8080808080808080ULL;
+  lo = (uint32_t)G;
+  hi = (uint32_t)(G >> 32);
 }
-// Two BF16 digits in one word: the upper halves of their (exact) FP32 images.
-__device__ __forceinline__ uint32_t bf16x2(float d0, float d1) {
-  return __byte_perm(__float_as_uint(d0), __float_as_uint(d1), 0x7632);
+// The same for E >= 64, in fewer integer instructions (they bound the slicing:
+// each takes its SM sub-partition's ALU pipe two cycles).  t = |x| 2^(1085 - E)
+// truncated (one bit more than F; 0 for zeros and subnormals, whose exponent
+// is at least 64 below E); with m the sign as a mask, (t ^ m) + 1 halves to F
+// rounded half away from zero for either sign, so G = ((t ^ m) + 1 + 2 C) >> 1
+// on 65 bits, C = 0x8080808080808080.
+__device__ __forceinline__ void offset_digits(double x, int E, uint32_t& lo, uint32_t& hi) {
+  const uint32_t xh = (uint32_t)__double2hiint(x), xl = (uint32_t)__double2loint(x);
+  const int k = min(E - (int)((xh >> 20) & 0x7ffu), 63);
+  const uint32_t th = (__funnelshift_l(xl, xh, 10) & 0x3fffffffu) | 0x40000000u;
+  const unsigned long long t = (((unsigned long long)th << 32) | (xl << 10)) >> k;
+  const uint32_t m = (uint32_t)((int)xh >> 31);
+  uint32_t s0, s1, s2;
+  asm("add.cc.u32 %0, %3, 0x01010101;\n\taddc.cc.u32 %1, %4, 0x01010101;\n\taddc.u32 %2, %5, 1;"
+      : "=r"(s0), "=r"(s1), "=r"(s2)
+      : "r"((uint32_t)t ^ m), "r"((uint32_t)(t >> 32) ^ m), "r"(m));
+  lo = __funnelshift_r(s0, s1, 1);
+  hi = __funnelshift_r(s1, s2, 1);
+}
+// Digit planes 0..G-1 of four values (consecutive K) as FP16 words, two values
+// each: store(p, words).  A byte b of G is the half 0x6400 | b = 1024 + b; less
+// 1152 it is the digit, exact in FP16.
+template <int G, class Store>
+__device__ __forceinline__ void quad_digits(double x0, double x1, double x2, double x3, int E, const Store& store) {
+  uint32_t w[4][2];
+  if (E >= 64) {
+    offset_digits(x0, E, w[0][0], w[0][1]);
+    offset_digits(x1, E, w[1][0], w[1][1]);
+    offset_digits(x2, E, w[2][0], w[2][1]);
+    offset_digits(x3, E, w[3][0], w[3][1]);
+  } else {
+    offset_digits_general(x0, E, w[0][0], w[0][1]);
+    offset_digits_general(x1, E, w[1][0], w[1][1]);
+    offset_digits_general(x2, E, w[2][0], w[2][1]);
+    offset_digits_general(x3, E, w[3][0], w[3][1]);
+  }
+  auto halves = [](uint32_t a, uint32_t b, int j) {   // byte j of a, of b
+    const uint32_t h = (__byte_perm(a, b, (uint32_t)(j | ((4 + j) << 8))) & 0x00ff00ffu) | 0x64006400u;
+    uint32_t d;
+    asm("sub.f16x2 %0, %1, %2;" : "=r"(d) : "r"(h), "r"(0x64806480u));
+    return d;
+  };
+#pragma unroll
+  for (int p = 0; p < G; p++) {
+    const int j = (kS - 1 - p) & 3, h = p < 4 ? 1 : 0;
+    uint2 v;
+    v.x = halves(w[0][h], w[1][h], j);
+    v.y = halves(w[2][h], w[3][h], j);
+    store(p, v);
+  }
 }
 // Byte offset of element (row, kk) (kk < 16) inside one K-major slice block:
 // core matrices [row/8][kk/8][8][16 bytes].
@@ -474,19 +512,9 @@ __device__ __forceinline__ void slice_b_quad(Ctx& c, uint8_t* stage, int g, int 
   // two 16-byte loads: conflict-free (a quarter warp covers all 8 16-byte bank groups)
   const double2* y = reinterpret_cast<const double2*>(c.sY + col * kLdY + k0 + 4 * q);
   const double2 y01 = y[0], y23 = y[1];
-  float d[4][kS];
-  digits(fixed_of(y01.x, E), d[0]);
-  digits(fixed_of(y01.y, E), d[1]);
-  digits(fixed_of(y23.x, E), d[2]);
-  digits(fixed_of(y23.y, E), d[3]);
-  const int off = core_off(col, 4 * q);
-#pragma unroll
-  for (int p = 0; p < G; p++) {
-    uint2 w;
-    w.x = bf16x2(d[0][p], d[1][p]);
-    w.y = bf16x2(d[2][p], d[3][p]);
-    *reinterpret_cast<uint2*>(stage + p * kSliceBBytes + off) = w;
-  }
+  uint8_t* dst = stage + core_off(col, 4 * q);
+  quad_digits<G>(y01.x, y01.y, y23.x, y23.y, E,
+                 [&](int p, uint2 w) { *reinterpret_cast<uint2*>(dst + p * kSliceBBytes) = w; });
 }
 
 __device__ __forceinline__ void mbar_arrive(uint64_t* b) {
@@ -542,7 +570,7 @@ inline __device__ bool gemm(Ctx& c, const uint8_t* X, const uint8_t* Xnext, int 
   bool ok = true;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   if (warp == 0) {
-    const uint32_t id = idesc_bf16(kM, kN);
+    const uint32_t id = idesc_f16(kM, kN);
     const uint64_t dA0 = sdesc(smem_u32(c.sA), 128, 256);
     const uint64_t dB0 = sdesc(smem_u32(c.sB), 128, 256);
     for (int j = 0; j < nch; j++) {
@@ -564,13 +592,13 @@ inline __device__ bool gemm(Ctx& c, const uint8_t* X, const uint8_t* Xnext, int 
           const uint64_t a = dA + (uint64_t)((p * kSliceABytes) >> 4), b = dB + (uint64_t)((q * kSliceBBytes) >> 4);
           const int last_q = G - 1 - p;   // slice p's last product
           if (last_q == 0)
-            mma_bf16<kARead>(d, a, b, id, acc);
+            mma_f16<kARead>(d, a, b, id, acc);
           else if (q == 0)
-            mma_bf16<kAFill>(d, a, b, id, acc);
+            mma_f16<kAFill>(d, a, b, id, acc);
           else if (q < last_q)
-            mma_bf16<kAUse>(d, a, b, id, acc);
+            mma_f16<kAUse>(d, a, b, id, acc);
           else
-            mma_bf16<kALast>(d, a, b, id, acc);
+            mma_f16<kALast>(d, a, b, id, acc);
         }
       }
       mma_commit(c.bar + kBarDone + n % kDoneStages);
@@ -634,16 +662,13 @@ inline __device__ bool gemm(Ctx& c, const uint8_t* X, const uint8_t* Xnext, int 
 //  * g_0..g_2 (|g| <= 2^22) come from the FP32 adder: the encoding of
 //    g + 1.5 2^23 is g plus a constant (removed once, in the sum); the others
 //    from the conversion unit.
-//  * V = hi 2^32 + lo (64-bit Horner chains over t < 4 and t >= 4), then
-//    V = vh 2^32 + vl with vl the low 32 bits of lo.
-//  * X = V / 2^s rounded to odd (truncated, last bit set when a discarded bit
-//    is), s the smallest shift that leaves |X| <= 2^62: when s > 0, X keeps 62
-//    significant bits, so rounding X to 53 bits is the correct rounding of V
-//    (rounding to odd at >= 55 bits makes the second rounding innocuous).
-//  * |X| normalised, rounded to 53 bits and placed in the IEEE 754 encoding
-//    with integer operations: on this part the FP64 pipe (which also converts
-//    integers to binary64) is scarce, and the epilogue keeps it for the one
-//    addition per element.
+//  * V = hi 2^32 + lo (64-bit Horner chains over t < 4 and t >= 4) as three
+//    32-bit words, then |V|: its leading one shifted to the top of two words
+//    and a remainder, rounded to 53 bits there, and placed in the IEEE 754
+//    encoding, all with 32-bit integer operations: on this part the FP64 pipe
+//    (which also converts integers to binary64) is scarce, and the epilogue
+//    keeps it for the one addition per element.  The integer ALU bounds it (two
+//    cycles an instruction and sub-partition).
 constexpr float kMagic = 12582912.0f;                                 // 1.5 2^23
 constexpr long long kMagicSum = 0x4B400000LL * (16777216LL + 65536LL + 256LL);
 __device__ __forceinline__ double recombine(const uint32_t (&acc)[kGroups][kDC], int i, int k,
@@ -659,27 +684,39 @@ __device__ __forceinline__ double recombine(const uint32_t (&acc)[kGroups][kDC],
   const long long hi = b0 * 16777216LL + b1 * 65536LL + b2 * 256LL + (g3 - kMagicSum);
   const long long lo = g4 * 16777216LL + g5 * 65536LL + g6 * 256LL + g7;
   const long long vh = hi + (lo >> 32);                  // |vh| < 2^45
-  const uint32_t vl = (uint32_t)lo;
-  // s = bit length of |vh| (one's complement for negatives) beyond 30 bits, in [0, 15]
-  const uint32_t top = (uint32_t)((unsigned long long)(vh ^ (vh >> 63)) >> 30);
-  const int s = 32 - __clz((int)top);
-  const uint32_t sticky = (uint32_t)((unsigned long long)vl << (32 - s)) != 0u ? 1u : 0u;
-  const long long X =
-      (long long)(((unsigned long long)vh << (32 - s)) | (unsigned long long)((vl >> s) | sticky));
-  const unsigned long long sg = (unsigned long long)(X >> 63);
-  const unsigned long long ax = ((unsigned long long)X ^ sg) - sg;   // |X| <= 2^62
-  const int lz = __clzll((long long)ax);                 // 64 when X == 0
-  const unsigned long long u = ax << (lz & 63);          // leading one at bit 63
-  const unsigned long long m = u >> 11;                  // 53 significant bits
-  const uint32_t low = (uint32_t)u & 0x7FFu;             // round half to even on the 11 dropped bits
-  const unsigned long long mr = m + (((low + ((uint32_t)m & 1u)) > 0x400u) ? 1ULL : 0ULL);
-  const int e = k + s + 1023 + 63 - lz;                  // biased exponent before a rounding carry
-  // m carries its leading one into the exponent field (a rounding carry to
+  uint32_t a2 = (uint32_t)(vh >> 32), a1 = (uint32_t)vh, a0 = (uint32_t)lo;
+  const uint32_t m = (uint32_t)((int)a2 >> 31);          // the sign as a mask
+  asm("sub.cc.u32 %0, %3, %6;\n\tsubc.cc.u32 %1, %4, %6;\n\tsubc.u32 %2, %5, %6;"
+      : "=r"(a0), "=r"(a1), "=r"(a2)
+      : "r"(a0 ^ m), "r"(a1 ^ m), "r"(a2 ^ m), "r"(m));   // |V|
+  int top = 95;                                          // weight of a2's top bit
+  if (a2 == 0u) {
+    a2 = a1;
+    a1 = a0;
+    a0 = 0u;
+    top = 63;
+  }
+  if (a2 == 0u) {
+    a2 = a1;
+    a1 = 0u;
+    top = 31;
+  }
+  const int lz = __clz((int)a2);
+  const uint32_t c2 = __funnelshift_lc(a1, a2, lz), c1 = __funnelshift_lc(a0, a1, lz), c0 = a0 << (lz & 31);
+  // 53 bits of c2:c1, the 11 bits below them and c0: round half to even
+  const uint32_t mh = c2 >> 11, ml = __funnelshift_r(c1, c2, 11);
+  const uint32_t rest = ((c1 & 0x7ffu) << 1) | (c0 != 0u ? 1u : 0u);
+  const uint32_t up = rest + (ml & 1u) > 0x800u ? 1u : 0u;
+  const int e = top - lz + k + 1023;                     // biased exponent before a rounding carry
+  // mh carries its leading one into the exponent field (a rounding carry to
   // 2^53 bumps the exponent once more, with a zero fraction)
-  const unsigned long long bits = mr + ((unsigned long long)(e - 1) << 52);
-  const unsigned long long res =
-      (!valid || ax == 0ULL || e < 1) ? 0ULL : (e > 2046 ? 0x7FF0000000000000ULL : bits);
-  return __longlong_as_double((long long)(res | (sg & 0x8000000000000000ULL)));
+  uint32_t rl, rh;
+  asm("add.cc.u32 %0, %2, %4;\n\taddc.u32 %1, %3, 0;" : "=r"(rl), "=r"(rh) : "r"(ml), "r"(mh + ((uint32_t)(e - 1) << 20)), "r"(up));
+  if (!valid || (int)c2 >= 0 || (unsigned)(e - 1) >= 2046u) {
+    rl = 0u;
+    rh = valid && (int)c2 < 0 && e > 2046 ? 0x7FF00000u : 0u;
+  }
+  return __hiloint2double((int)(rh | (m & 0x80000000u)), (int)rl);
 }
 
 // Epilogue modes (R = the product just computed).
@@ -781,18 +818,9 @@ inline __device__ void slice_cols(const Acc& acc, uint8_t* dst, const int* sE, i
     const int r = qd % kK;
     const int k4 = (qd / kK) * 4;
     const int E = sE[r];
-    float d[4][kS];
-#pragma unroll
-    for (int i = 0; i < 4; i++) digits(fixed_of(acc(r, k4 + i), E), d[i]);
-    uint8_t* blk = dst + (size_t)(k4 / kKC) * kAChunkBytes;
-    const int off = core_off(r, k4 % kKC);
-#pragma unroll
-    for (int p = 0; p < kS; p++) {
-      uint2 w;
-      w.x = bf16x2(d[0][p], d[1][p]);
-      w.y = bf16x2(d[2][p], d[3][p]);
-      *reinterpret_cast<uint2*>(blk + p * kSliceABytes + off) = w;
-    }
+    uint8_t* blk = dst + (size_t)(k4 / kKC) * kAChunkBytes + core_off(r, k4 % kKC);
+    quad_digits<kS>(acc(r, k4), acc(r, k4 + 1), acc(r, k4 + 2), acc(r, k4 + 3), E,
+                    [&](int p, uint2 w) { *reinterpret_cast<uint2*>(blk + p * kSliceABytes) = w; });
   }
   fence_proxy_async_global();
   __syncthreads();
