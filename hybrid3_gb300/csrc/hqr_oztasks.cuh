@@ -41,56 +41,111 @@ struct PackedTAcc {
 
 // T recurrence (dlarft 'F','C', k = NB = 128) in shared memory,
 //   T(c, c) = tau_c;  T(0:c, c) = -tau_c T(0:c, 0:c) G(0:c, c)  (zero when tau_c = 0),
-// regrouped by blocks of 16 columns: first the diagonal 16 x 16 blocks (each
-// row runs its own scalar recurrence over its own row: no barrier), then for
-// block columns b = 1..7
-//   X = G(0:bw, bw:bw+16) T_bb,   T(0:bw, bw:bw+16) = -T(0:bw, 0:bw) X,
-// the same sums (tau_c = 0 leaves column c zero either way).  FP64 on this
-// part issues one warp instruction per ~19 cycles per SM, so the work is laid
-// out for full warps: the triangular product pairs rows r and bw-1-r, whose
-// dots add up to bw + 1 terms.  The scalar column recurrence left most lanes
-// of a warp idle on the short rows and took 2.6x longer.
+// by doubling: first the diagonal 16 x 16 blocks (each row runs its own scalar
+// recurrence over its own row: no barrier), then for H = 16, 32, 64 the block
+// of every pair of neighbouring H x H diagonal blocks,
+//   T12 = -T11 (G12 T22),
+// the same sums regrouped (tau_c = 0 leaves column c zero either way).  The
+// FP64 pipe bounds it (an FMA of a warp per 16 cycles of the SM; 350 kFMA are
+// 178 kcycles), so each product is laid out for full warps that skip the
+// triangle's zeros: the lanes run along the dense side, a thread's H / 4 sums
+// along the triangular one, four apart, which gives every warp the same work,
+// four of them at a time: loops whose bodies need no branch per term keep the
+// loads ahead of the FMAs (all H / 4 sums at once with a branch per term took
+// 403 kcycles).  210 kcycles; by block columns of 16 it took 310.
 // sG: strictly upper part of G = V^T V, packed: G(b, c) (b < c) at c (c - 1) / 2 + b.
 // sT: the result, packed upper: T(a, b) (a <= b) at b (b + 1) / 2 + a.
-// sX: (NB - 16) x 16 doubles of scratch.
+// sX: 64 x kLdX doubles of scratch.
+constexpr int kLdX = 65;
+// Sixteen terms of four sums: acc[i] += x(d) y(d, i), d = 0..15; with DIAG only
+// the terms of a triangular block, d <= 4 i + res (UPPER) or d >= 4 i + res.
+template <bool DIAG, bool UPPER, class X, class Y>
+__device__ __forceinline__ void t_terms(double (&acc)[4], int res, X x, Y y) {
+#pragma unroll
+  for (int d = 0; d < 16; d++) {
+    const double xd = x(d);
+#pragma unroll
+    for (int i = 0; i < 4; i++) {
+      if (DIAG && (UPPER ? i < d / 4 : i > d / 4)) continue;
+      const double yd = y(d, i);
+      const bool in = !DIAG || i != d / 4 || (UPPER ? d % 4 <= res : d % 4 >= res);
+      acc[i] = fma(in ? xd : 0.0, in ? yd : 0.0, acc[i]);
+    }
+  }
+}
+template <int H>
+__device__ __forceinline__ void t_double(const double* sG, double* sT, double* sX) {
+  constexpr int L = H < 32 ? H : 32, NB = H / 16;
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  // the pair of blocks, this lane's dense index, this thread's residue mod 4
+  const int pair = H == 64 ? 0 : H == 32 ? w >> 2 : w >> 1;
+  const int dense = (H == 64 ? (w & 1) * 32 : 0) + lane % L;
+  const int res = H == 64 ? w >> 1 : H == 32 ? w & 3 : (w & 1) * 2 + lane / L;
+  const int b1 = pair * 2 * H, b2 = b1 + H;
+  double* X = sX + pair * H;   // (the pairs' columns side by side: H * pairs = 64)
+  auto T = [&](int a, int b) -> double& { return sT[b * (b + 1) / 2 + a]; };
+  // X(r, j) = sum_{d <= j} G12(r, d) T22(d, j): r = dense, j = 16 jb + 4 i + res
+#pragma unroll 1
+  for (int jb = 0; jb < NB; jb++) {
+    double acc[4] = {0.0, 0.0, 0.0, 0.0};
+    auto g = [&](int db) {
+      return [=](int d) { const int c = b2 + 16 * db + d; return sG[c * (c - 1) / 2 + b1 + dense]; };
+    };
+    auto t = [&](int db) {
+      return [=](int d, int i) { return T(b2 + 16 * db + d, b2 + 16 * jb + 4 * i + res); };
+    };
+#pragma unroll 1
+    for (int db = 0; db < jb; db++) t_terms<false, true>(acc, res, g(db), t(db));
+    t_terms<true, true>(acc, res, g(jb), t(jb));
+#pragma unroll
+    for (int i = 0; i < 4; i++) X[dense * kLdX + 16 * jb + 4 * i + res] = acc[i];
+  }
+  __syncthreads();
+  // T12(r, j) = -sum_{d >= r} T11(r, d) X(d, j): j = dense, r = 16 rb + 4 i + res
+#pragma unroll 1
+  for (int rb = 0; rb < NB; rb++) {
+    double acc[4] = {0.0, 0.0, 0.0, 0.0};
+    auto x = [&](int db) { return [=](int d) { return X[(16 * db + d) * kLdX + dense]; }; };
+    auto t = [&](int db) {
+      return [=](int d, int i) { return T(b1 + 16 * rb + 4 * i + res, b1 + 16 * db + d); };
+    };
+    t_terms<true, false>(acc, res, x(rb), t(rb));
+#pragma unroll 1
+    for (int db = rb + 1; db < NB; db++) t_terms<false, false>(acc, res, x(db), t(db));
+#pragma unroll
+    for (int i = 0; i < 4; i++) T(b1 + 16 * rb + 4 * i + res, b2 + dense) = -acc[i];
+  }
+  __syncthreads();
+}
 inline __device__ void t_recurrence(const double* sG, double* sT, double* sX, const double* tau) {
   constexpr int K = oz::kK, BS = 16;
   const int tid = threadIdx.x;
   if (tid < K) {
+    // row `tid` of its block: every T(tid, d) goes to the sums of the later columns
     const int b = tid / BS, a = tid % BS;
-    for (int c = a; c < BS; c++) {
-      const int gc = b * BS + c;
-      const double tc = __ldcg(tau + gc);
-      double s = 0.0;
-      for (int d = a; d < c; d++) {
-        const int gd = b * BS + d;
-        s = fma(sT[gd * (gd + 1) / 2 + tid], sG[gc * (gc - 1) / 2 + gd], s);
+    const double my_tau = __ldcg(tau + tid);
+    double acc[BS];
+#pragma unroll
+    for (int c = 0; c < BS; c++) acc[c] = 0.0;
+#pragma unroll
+    for (int d = 0; d < BS; d++) {
+      const int gd = b * BS + d;
+      const double td = __shfl_sync(0xffffffffu, my_tau, d, BS);
+      if (d >= a) {
+        const double t = d == a ? td : td == 0.0 ? 0.0 : -td * acc[d];
+        sT[gd * (gd + 1) / 2 + tid] = t;
+#pragma unroll
+        for (int c = d + 1; c < BS; c++) {
+          const int gc = b * BS + c;
+          acc[c] = fma(t, sG[gc * (gc - 1) / 2 + gd], acc[c]);
+        }
       }
-      sT[gc * (gc + 1) / 2 + tid] = (c == a) ? tc : (tc == 0.0 ? 0.0 : -tc * s);
     }
   }
   __syncthreads();
-  for (int b = 1; b < K / BS; b++) {
-    const int bw = b * BS;
-    for (int e = tid; e < bw * BS; e += kThreads) {
-      const int r = e % bw, j = e / bw;
-      double s = 0.0;
-      for (int d = 0; d <= j; d++)
-        s = fma(sG[(bw + d) * (bw + d - 1) / 2 + r], sT[(bw + j) * (bw + j + 1) / 2 + bw + d], s);
-      sX[r + j * bw] = s;
-    }
-    __syncthreads();
-    for (int e = tid; e < (bw / 2) * BS; e += kThreads) {
-      const int r0 = e % (bw / 2), j = e / (bw / 2), r1 = bw - 1 - r0;
-      double s0 = 0.0, s1 = 0.0;
-      for (int d = r0; d < bw; d++) s0 = fma(sT[d * (d + 1) / 2 + r0], sX[d + j * bw], s0);
-      for (int d = r1; d < bw; d++) s1 = fma(sT[d * (d + 1) / 2 + r1], sX[d + j * bw], s1);
-      const int cj = bw + j;
-      sT[cj * (cj + 1) / 2 + r0] = -s0;
-      sT[cj * (cj + 1) / 2 + r1] = -s1;
-    }
-    __syncthreads();
-  }
+  t_double<16>(sG, sT, sX);
+  t_double<32>(sG, sT, sX);
+  t_double<64>(sG, sT, sX);
 }
 
 // Shape of a panel tile's reflectors V.
@@ -145,16 +200,25 @@ inline __device__ bool task_ozprep(const double* V, const double* tau, double* G
   double* sT = sG + kK * (kK - 1) / 2;
   int* sE = reinterpret_cast<int*>(sT + kK * (kK + 1) / 2);
   double* sX = reinterpret_cast<double*>(sE + kK);
-  static_assert((kK * (kK - 1) / 2 + kK * (kK + 1) / 2) * 8 + kK * 4 + (kK - 16) * 16 * 8 <= kSmemBytes,
+  static_assert((kK * (kK - 1) / 2 + kK * (kK + 1) / 2) * 8 + kK * 4 + 64 * kLdX * 8 <= kSmemBytes,
                 "T recurrence scratch");
-  constexpr int kPacked = kK * (kK - 1) / 2;
-#pragma unroll 4
-  for (int idx = threadIdx.x; idx < kPacked; idx += kThreads) {
-    // column c of packed index idx: c (c - 1) / 2 <= idx < (c + 1) c / 2
-    int c = (int)((1.0f + sqrtf(1.0f + 8.0f * (float)idx)) * 0.5f);
-    while (c * (c - 1) / 2 > idx) c--;
-    while ((c + 1) * c / 2 <= idx) c++;
-    sG[idx] = __ldcg(G + (idx - c * (c - 1) / 2) + (size_t)c * kK);
+  // a warp packs 16 columns, four columns' loads in flight
+  for (int c0 = threadIdx.x >> 5; c0 < kK; c0 += 4 * kWarps) {
+    double v[4][kK / 32];
+#pragma unroll
+    for (int i = 0; i < 4; i++)
+#pragma unroll
+      for (int q = 0; q < kK / 32; q++) {
+        const int c = c0 + i * kWarps, r = 32 * q + (threadIdx.x & 31);
+        v[i][q] = r < c ? __ldcg(G + r + (size_t)c * kK) : 0.0;
+      }
+#pragma unroll
+    for (int i = 0; i < 4; i++)
+#pragma unroll
+      for (int q = 0; q < kK / 32; q++) {
+        const int c = c0 + i * kWarps, r = 32 * q + (threadIdx.x & 31);
+        if (r < c) sG[c * (c - 1) / 2 + r] = v[i][q];
+      }
   }
   __syncthreads();
   t_recurrence(sG, sT, sX, tau);
