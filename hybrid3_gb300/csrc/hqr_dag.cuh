@@ -857,12 +857,16 @@ __global__ void __launch_bounds__(kThreads, BATCH ? 2 : 1) dag_exec_kernel(DagPa
       task_ozprep(prep_v, prep_tau, prep_g, prep_kind, prep_slices, prep_exps, reinterpret_cast<uint8_t*>(smem),
                   s_tmem, q.ctl + kErr, !applies_h(q.mode));
     if (OZ && oz_bot) {
-      for (int cc = 0; cc < q.oz_cpt; cc++) {
-        if (q.c_cols > 0 && oz_col0 + (long long)cc * oz::kN >= q.c_cols) break;
+      int chunks = q.oz_cpt;
+      if (q.c_cols > 0) chunks = (int)min((long long)chunks, (q.c_cols - oz_col0 + oz::kN - 1) / oz::kN);
+      // one set-up of the engine for all of them (a set-up each for the reduced
+      // products: 50.7 us a task of two, 52.1 with one)
+      const int per = OZG == oz::kGroups ? chunks : 1;
+      for (int cc = 0; cc < chunks; cc += per) {
         const size_t co = (size_t)cc * oz::kN * NB;
         oz::Ctx c;
         oz::ctx_init(c, reinterpret_cast<uint8_t*>(smem), s_tmem, q.ctl + kErr);
-        if (!task_ozapply<OZG>(c, oz_slices, oz_exps, oz_top ? oz_top + co : nullptr, oz_bot + co)) break;
+        if (!task_ozapply<OZG>(c, oz_slices, oz_exps, oz_top ? oz_top + co : nullptr, oz_bot + co, per)) break;
       }
     }
     fence_acq_rel_gpu();   // release: this task's writes before its dependents' counters

@@ -266,25 +266,30 @@ inline __device__ bool task_ozprep(const double* V, const double* tau, double* G
   return true;
 }
 
-// One 64-column block of the update.  Ctop: A1 block (SSRFB) or nullptr
-// (LARFB); Cbot: A2 block (SSRFB) or the C block (LARFB); ld NB.  Returns
-// false on a device time-out (error word already set).  G: t-groups of the
-// products (8: FP64-level; 4: the reduced form, see oz::product).
+// `chunks` 64-column blocks of the update, one after the other.  Ctop: A1 block
+// (SSRFB) or nullptr (LARFB); Cbot: A2 block (SSRFB) or the C block (LARFB); ld
+// NB.  Returns false on a device time-out (error word already set).  G: t-groups
+// of the products (8: FP64-level; 4: the reduced form, see oz::product).
 template <int G = oz::kGroups>
 inline __device__ bool task_ozapply(oz::Ctx& c, const uint8_t* slices, const int* exps, double* Ctop,
-                                    double* Cbot) {
+                                    double* Cbot, int chunks) {
   using namespace oz;
   constexpr size_t ob = operand_bytes();
   const uint8_t* X1 = slices + kOzX * ob;
   const uint8_t* XV = slices + kOzV * ob;
   prefetch<G>(c, X1);
-  // the right operand [C_bot; C_top]: C_bot staged, C_top loaded after chunk 7;
-  // column exponents over both
-  stage_y(c, Cbot, kK, -1, false, Ctop);
-  if (!product<G>(c, X1, XV, exps + kOzX * kK, kEpiToYSubTop, nullptr, 0, Ctop, kK,
-                  Ctop ? 2 * kChunks : kChunks, Ctop))
-    return false;
-  if (!product<G>(c, XV, nullptr, exps + kOzV * kK, kEpiSubInto, Cbot, kK, nullptr, 0)) return false;
+  for (int cc = 0; cc < chunks; cc++) {
+    // the right operand [C_bot; C_top]: C_bot staged, C_top loaded after chunk 7;
+    // column exponents over both
+    stage_y(c, Cbot, kK, -1, false, Ctop);
+    if (!product<G>(c, X1, XV, exps + kOzX * kK, kEpiToYSubTop, nullptr, 0, Ctop, kK, Ctop ? 2 * kChunks : kChunks,
+                    Ctop))
+      return false;
+    if (!product<G>(c, XV, cc + 1 < chunks ? X1 : nullptr, exps + kOzV * kK, kEpiSubInto, Cbot, kK, nullptr, 0))
+      return false;
+    Cbot += kN * kK;
+    if (Ctop) Ctop += kN * kK;
+  }
   ctx_release(c);
   return true;
 }
