@@ -187,19 +187,37 @@ static int run_dag(DagParams& p, DagWorkspace* ws, const Geometry& g, cudaStream
 // -> 28.4 ms; split n = 16384 unchanged.  FP32 panels have no such steps: their
 // blocks take half the time and are latency, not work (32768 x 8192: 355 ms
 // with none, 356 from 300 tiles on, 382 from 6000).
+//
+// Such a task takes a part of a block's w columns: the chain through a tile is
+// its panel blocks and the first part after each, and a part of 8 / 16 / 32
+// columns takes 52 / 84 / 156 us at tile order 256 (8 / 16: 13 / 22 us at 128).
+// Parts of 8 cost a third more work than blocks of 32, so they are taken where
+// there are at most two panel tiles to an SM (factorization, ms, parts of 8 /
+// 16 / whole blocks: FP64 n = 2048, NB 256: 25.7 / 27.2 / 31.4, n = 4096: 112.2
+// / 113.4 / 116.9; 1000 x 615, NB 96, with its solve: 6.53 / 6.87 / 7.59; split
+// n = 3072: 21.4 / - / 22.2; but 594 panel tiles: FP64 38400 x 1024, NB 256:
+// 118 / 112.2 / 111.8, split 19200 x 512: 18.2 / - / 14.6), and FP64 parts of
+// 16 beyond that.
 struct FineSteps {
-  int from = 0;
+  int from = 0, sub = 1;
   long long ids = 0, tasks = 0;
 };
 constexpr long long kFineTilesSplit = 6000, kFineTilesFp64 = 600, kFineTilesFp32 = 0;
-static FineSteps fine_steps(const Geometry& g, bool split, bool fp32 = false) {
+static FineSteps fine_steps(const Geometry& g, bool split, bool fp32 = false, bool parts = true) {
   FineSteps f;
   const long long nblk = g.NB / g.w, tiles = fp32 ? kFineTilesFp32 : split ? kFineTilesSplit : kFineTilesFp64;
   while (f.from < g.steps && (long long)(g.NT - f.from - 1) * (g.MT - f.from - 1) > tiles) f.from++;
   if (nblk < 2) return f;
-  f.ids = (long long)(g.steps - f.from) * g.MT * nblk * nblk;
-  for (int i = f.from; i < g.steps; i++) f.tasks += (g.MT - i) * nblk * (nblk - 1) / 2;
-  if ((long long)coarse_task_ids(g, split ? 2 : g.NC) + f.ids > 0x3fffffffLL) f.ids = f.tasks = 0;
+  long long panels = 0;
+  for (int i = f.from; i < g.steps; i++) panels += g.MT - i;
+  const int part = panels <= 2LL * dag_sm_count() && !fp32 ? 8 : split ? g.w : 16;
+  if (parts && g.w % part == 0) f.sub = g.w / part;
+  f.ids = (long long)(g.steps - f.from) * g.MT * nblk * nblk * f.sub;
+  for (int i = f.from; i < g.steps; i++) f.tasks += (g.MT - i) * nblk * (nblk - 1) / 2 * f.sub;
+  if ((long long)coarse_task_ids(g, split ? 2 : g.NC) + f.ids > 0x3fffffffLL) {
+    if (f.sub > 1) return fine_steps(g, split, fp32, false);
+    f.ids = f.tasks = 0;
+  }
   return f;
 }
 
@@ -252,9 +270,14 @@ static FactorTasks factor_tasks(const Geometry& g) {
   for (int i = 0; i < g.steps; i++) tiles += (long long)(g.NT - 1 - i) * (g.MT - i);
   FactorTasks f{update_columns(g, tiles, g.MT + g.steps, g.NB), fine_steps(g, false), 0};
   f.ids = coarse_task_ids(g, g.NB / f.cb) + (size_t)f.fine.ids;
-  if (external_bytes(g, coarse_task_ids(g, g.NC)) <= kNoAllocScratchBytes &&
-      external_bytes(g, f.ids) > kNoAllocScratchBytes)
-    f = FactorTasks{g.CB, FineSteps{}, coarse_task_ids(g, g.NC)};
+  if (external_bytes(g, coarse_task_ids(g, g.NC)) <= kNoAllocScratchBytes) {
+    if (f.fine.sub > 1 && external_bytes(g, f.ids) > kNoAllocScratchBytes) {
+      f.fine = fine_steps(g, false, false, false);
+      f.ids = coarse_task_ids(g, g.NB / f.cb) + (size_t)f.fine.ids;
+    }
+    if (external_bytes(g, f.ids) > kNoAllocScratchBytes)
+      f = FactorTasks{g.CB, FineSteps{}, coarse_task_ids(g, g.NC)};
+  }
   return f;
 }
 
@@ -332,6 +355,7 @@ int launch_factor(const Geometry& g, DagWorkspace* ws, double* dA, double* dT, d
   set_columns(p, g, cb, g.NB);
   p.fine_from = fine.from;
   p.fine_ids = (int)fine.ids;
+  p.fine_sub = fine.sub;
   // tasks: per step i, nblk inner blocks of each of the MT-i panel tiles [+ one
   // OZPREP per panel tile] + NC*(NT-1-i)*(MT-i) updates; a tree adds per merge
   // nblk blocks [+ one OZPREP] + NC*(NT-1-i) merge updates; a fine step nblk
@@ -655,6 +679,7 @@ int launch_factor_external(const Geometry& g, const ExternalScratch& x, double* 
   p.sp = SmemPlan::make(p.sh);
   p.fine_from = fine.from;
   p.fine_ids = (int)fine.ids;
+  p.fine_sub = fine.sub;
   p.n_ids = (int)f.ids;
   long long n = fine.tasks;
   for (int i = 0; i < g.steps; i++)

@@ -115,9 +115,9 @@ struct DagParams {
   int* cnt;         // dependency counters, one per task id
   // Factorization with the flat tree, fine_ids > 0: in the steps from
   // fine_from on, a panel block (GEQRT or TSQRT inner block b of tile k) is its
-  // column loop only; its trailing update is one task per later w-column block
-  // j of the tile (fine_ids task ids).
-  int fine_from, fine_ids;
+  // column loop only; its trailing update is one task per part j of the tile's
+  // later columns (fine_ids task ids), fine_sub parts to a block of w columns.
+  int fine_from, fine_ids, fine_sub;
   int* qhi;         // ready FIFOs, capacity n_ids each
   int* qlo;
   unsigned* ctl;
@@ -170,7 +170,8 @@ __host__ __device__ __forceinline__ bool is_top(const DagParams& p, int i, int k
 //   merge  (i, d, b)     : M0 + (i*dmax + d)*nblk + b            (1 <= d < domains)
 //   merge prep (i, d)    : Q0 + i*dmax + d     (split precision)
 //   merge update (i, j, d, c): X0 + ((i*J + j)*dmax + d)*NC + c
-//   trailing (i, k, b, j): Y0 + (((i - fine_from)*MT + k)*nblk + b)*nblk + j   (j > b, i >= fine_from)
+//   trailing (i, k, b, j): Y0 + (((i - fine_from)*MT + k)*nblk + b)*nblk*fine_sub + j
+//                          (j / fine_sub > b, i >= fine_from)
 __host__ __device__ __forceinline__ int panel_id(const DagParams& p, int i, int k, int b = 0) {
   return (i * p.MT + k) * p.nblk + b;
 }
@@ -208,7 +209,7 @@ __host__ __device__ __forceinline__ int trail_base(const DagParams& p) {
   return ttmqr_base(p) + p.steps * p.J * p.dmax * p.NC;
 }
 __host__ __device__ __forceinline__ int trail_id(const DagParams& p, int i, int k, int b, int j) {
-  return trail_base(p) + (((i - p.fine_from) * p.MT + k) * p.nblk + b) * p.nblk + j;
+  return trail_base(p) + (((i - p.fine_from) * p.MT + k) * p.nblk + b) * (p.nblk * p.fine_sub) + j;
 }
 __host__ __device__ __forceinline__ bool fine_step(const DagParams& p, int i) {
   return p.fine_ids > 0 && i >= p.fine_from;
@@ -224,7 +225,7 @@ __host__ __device__ __forceinline__ size_t panel_slot(int MT, int i, int k) {
 }
 
 struct TaskDesc {
-  int type, i, j, k, c;   // c: column block of an update, inner block of a panel task (kTRAIL: j its column block)
+  int type, i, j, k, c;   // c: column block of an update, inner block of a panel task (kTRAIL: j its part of the columns)
 };
 
 __device__ __forceinline__ TaskDesc decode(const DagParams& p, int id) {
@@ -280,7 +281,7 @@ __device__ __forceinline__ TaskDesc decode(const DagParams& p, int id) {
     t.type = kTTMQR;
   } else {
     int u = id - trail_base(p);
-    t.j = u % p.nblk; u /= p.nblk;
+    t.j = u % (p.nblk * p.fine_sub); u /= p.nblk * p.fine_sub;
     t.c = u % p.nblk; u /= p.nblk;
     t.k = u % p.MT;
     t.i = p.fine_from + u / p.MT;
@@ -416,10 +417,10 @@ __device__ int init_deps(const DagParams& p, int id) {
     if (k >= i && !p.skip_panels) {
       // block 0: the previous step's update of the tile (NC column blocks);
       // block b > 0: block b - 1 of the same tile (in a fine step: its trailing
-      // update of column block b); a TSQRT block also waits for the same block
+      // updates of column block b's parts); a TSQRT block also waits for the same block
       // of the tile above (its domain top's rows of R)
       if (p.mode == kModeFactor)
-        deps = (b == 0 ? (i > 0 ? p.NC : 0) : 1) + (is_top(p, i, k) ? 0 : 1);
+        deps = (b == 0 ? (i > 0 ? p.NC : 0) : fine_step(p, i) ? p.fine_sub : 1) + (is_top(p, i, k) ? 0 : 1);
       else
         deps = 0;
     }
@@ -454,7 +455,7 @@ __device__ int init_deps(const DagParams& p, int id) {
     // trailing (i, k, b, j): panel block b of the tile; the earlier block's
     // update of the same columns; the tile above's update of R's rows
     int u = id - trail_base(p);
-    const int j = u % p.nblk; u /= p.nblk;
+    const int j = u % (p.nblk * p.fine_sub) / p.fine_sub; u /= p.nblk * p.fine_sub;
     const int b = u % p.nblk; u /= p.nblk;
     const int k = u % p.MT, i = p.fine_from + u / p.MT;
     if (k >= i && j > b) deps = 1 + (b > 0 ? 1 : 0) + (k > i ? 1 : 0);
@@ -603,7 +604,7 @@ __device__ bool release_dependents(const DagParams& p, const TaskDesc& t, int* k
       // the domain, or, from a domain's last tile, of the domain's merge
       const int d = dom_of(p, t.i, t.k);
       if (fine_step(p, t.i)) {
-        for (int j = t.c + 1; j < p.nblk; j++) release(p, trail_id(p, t.i, t.k, t.c, j));
+        for (int j = (t.c + 1) * p.fine_sub; j < p.nblk * p.fine_sub; j++) release(p, trail_id(p, t.i, t.k, t.c, j));
       } else if (t.c + 1 < p.nblk) {
         release(p, panel_id(p, t.i, t.k, t.c + 1));
       }
@@ -624,7 +625,7 @@ __device__ bool release_dependents(const DagParams& p, const TaskDesc& t, int* k
     return true;
   }
   if (t.type == kTRAIL) {
-    release(p, t.j == t.c + 1 ? panel_id(p, t.i, t.k, t.j) : trail_id(p, t.i, t.k, t.c + 1, t.j));
+    release(p, t.j / p.fine_sub == t.c + 1 ? panel_id(p, t.i, t.k, t.c + 1) : trail_id(p, t.i, t.k, t.c + 1, t.j));
     if (t.k + 1 < p.MT) release(p, trail_id(p, t.i, t.k + 1, t.c, t.j));
     return true;
   }
@@ -784,7 +785,7 @@ __global__ void __launch_bounds__(kThreads, BATCH ? 2 : 1) dag_exec_kernel(DagPa
         const size_t o = tile_off(t.k, t.i, q.MT, NB);
         if (!BATCH)
           task_trailing<PanelT>(q.A + tile_off(t.i, t.i, q.MT, NB), t.k > t.i ? q.A + o : nullptr, q.T + o, q.sh,
-                                smem, q.sp, t.c, t.j);
+                                smem, q.sp, t.c, t.j * (q.sh.w / q.fine_sub), q.sh.w / q.fine_sub);
         break;
       }
       case kTBUILD: {

@@ -1031,19 +1031,19 @@ __device__ void task_tsqrt_blk(double* A1, double* A2, double* T, double* tau_g,
   __syncthreads();
 }
 
-// Columns [j w, (j+1) w) of the trailing update of inner block b of a panel
+// Columns [cbeg, cbeg + cols) of the trailing update of inner block b of a panel
 // tile, as a task of its own: of a GEQRT (A2 null: V and C in the tile A1, on
 // rows >= b w) or of a TSQRT (rows [b w, (b+1) w) of R in A1, all of A2).
 template <typename RT = double>
 __device__ void task_trailing(double* A1, double* A2, const double* T, const TileShape& sh, double* smem,
-                              const SmemPlan& sp, int b, int j) {
+                              const SmemPlan& sp, int b, int cbeg, int cols) {
   const int NB = sh.NB, w = sh.w;
   RT* sm = reinterpret_cast<RT*>(smem);
   const int i0 = b * w;
   const int m = A2 ? NB : NB - i0;
   const double* V = A2 ? A2 + (size_t)i0 * NB : A1 + i0 + (size_t)i0 * NB;
-  for (int c0 = j * w; c0 < (j + 1) * w; c0 += sh.CB) {
-    const int ncol = min(sh.CB, (j + 1) * w - c0);
+  for (int c0 = cbeg; c0 < cbeg + cols; c0 += sh.CB) {
+    const int ncol = min(sh.CB, cbeg + cols - c0);
     RT* sCt = sm + sp.off_c1;                                // the w x ncol rows of R (GEQRT: with the rows below)
     RT* sCb = A2 ? sCt + w * sh.CB : sCt + w;
     const int ldt = A2 ? w : NB;

@@ -1,7 +1,7 @@
 """FP64 update tasks narrower than a tile's nominal column block, and panel
 blocks whose trailing updates are tasks: where the rules that choose them turn
-(one tile, one tile row, few tiles, a tile column with few right-hand sides),
-the results are the oracle's and the statistics count what they did before.
+(one tile, one tile row, few tiles, a tile column with few right-hand sides,
+few and many panel tiles), the results are the oracle's and the statistics count what they did before.
 
 Bar: n eps ||.||_F elementwise, as test_gpu_qr.py.
 """
@@ -17,6 +17,8 @@ EPS = np.finfo(np.float64).eps
 @pytest.mark.parametrize("M,N,NB,IB", [
     (64, 64, 64, 16), (128, 128, 64, 64), (192, 64, 64, 16), (64, 192, 64, 16), (480, 288, 96, 32), (288, 288, 48, 24),
     (640, 640, 128, 32), (1024, 512, 256, 32), (512, 512, 512, 32), (1280, 1280, 32, 8), (1536, 1536, 64, 16),
+    # parts of a block's trailing update: 24 columns in three, 32 in four up to two panel tiles an SM, in two beyond
+    (144, 96, 48, 24), (96, 96, 32, 32), (64 * 152, 128, 64, 32), (64 * 153, 128, 64, 32), (64 * 160, 128, 64, 32),
 ])
 def test_factor_and_apply(M, N, NB, IB):
     torch = pytest.importorskip("torch")
