@@ -39,7 +39,7 @@ METRIC = "tile-QR TFLOP/s at FP64-level backward error: split-precision vs plain
 DP = ctypes.POINTER(ctypes.c_double)
 
 
-PRECISION_TEXT = {"split": "split (Ozaki BF16 slices on tcgen05, FP64 panels)",
+PRECISION_TEXT = {"split": "split (Ozaki FP16 slices on tcgen05, FP64 panels)",
                   "fast": "reduced split (the 10 slice products of weight <= 3 on tcgen05, FP64 panels)",
                   "fp32": "FP32-class (FP32 panel arithmetic, the reduced split updates)",
                   "fp64": "fp64 (plain)"}

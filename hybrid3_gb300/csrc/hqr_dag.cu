@@ -286,8 +286,8 @@ static FactorTasks factor_tasks(const Geometry& g) {
 // scheduling round trips (a queue claim and the dependents' releases, about 6
 // us per task).  One, where the longest chain of whole-tile updates (`path`
 // tasks) takes longer than all `tiles` of them on every SM: the chain's time
-// halves (Q^T C and Q C, n = 8192, 512 columns: 21.5 -> 13.3 ms together).  C with data in one
-// chunk only (ccols) has nothing to cut.
+// halves (Q^T C and Q C, n = 8192, 512 columns: 21.5 -> 13.3 ms together, now
+// 11.4).  C with data in one chunk only (ccols) has nothing to cut.
 static int oz_chunks(long long tiles, long long path, long long ccols = 0) {
   return (ccols > 0 && ccols <= oz::kN) || tiles >= path * dag_sm_count() ? 2 : 1;
 }
