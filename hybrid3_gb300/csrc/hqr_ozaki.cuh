@@ -839,17 +839,26 @@ inline __device__ bool product(Ctx& c, const uint8_t* Xprep, const uint8_t* Xnex
 // ---------------------------------------------------------------------------
 // Columns k < kcount of X(r, k) = acc(r, k) (kcount a multiple of kKC) into
 // dst in the [kc][slice][core layout] order, with the row exponents sE
-// (shared) already known.
+// (shared) already known.  Eight values a step: a row of a core matrix, so
+// that a warp's 16-byte stores fill whole sectors (a panel tile's five passes
+// through here: 90 -> 70 kcycles; with 8-byte stores, half a sector each, requesting
+// the next values ahead gained nothing).
 template <class Acc>
 inline __device__ void slice_cols(const Acc& acc, uint8_t* dst, const int* sE, int kcount) {
-  const int quads = kK * kcount / 4;
-  for (int qd = threadIdx.x; qd < quads; qd += kThreads) {
-    const int r = qd % kK;
-    const int k4 = (qd / kK) * 4;
-    const int E = sE[r];
-    uint8_t* blk = dst + (size_t)(k4 / kKC) * kAChunkBytes + core_off(r, k4 % kKC);
-    quad_digits<kS>(acc(r, k4), acc(r, k4 + 1), acc(r, k4 + 2), acc(r, k4 + 3), E,
-                    [&](int p, uint2 w) { *reinterpret_cast<uint2*>(blk + p * kSliceABytes) = w; });
+  static_assert(kThreads % kK == 0, "rows");
+  const int r = threadIdx.x % kK;   // the same row in all of a thread's steps
+  const int E = sE[r];
+  for (int k8 = threadIdx.x / kK * 8; k8 < kcount; k8 += kThreads / kK * 8) {
+    uint8_t* blk = dst + (size_t)(k8 / kKC) * kAChunkBytes + core_off(r, k8 % kKC);
+    double x[8];
+#pragma unroll
+    for (int i = 0; i < 8; i++) x[i] = acc(r, k8 + i);
+    uint2 lo[kS], hi[kS];
+    quad_digits<kS>(x[0], x[1], x[2], x[3], E, [&](int p, uint2 w) { lo[p] = w; });
+    quad_digits<kS>(x[4], x[5], x[6], x[7], E, [&](int p, uint2 w) { hi[p] = w; });
+#pragma unroll
+    for (int p = 0; p < kS; p++)
+      *reinterpret_cast<uint4*>(blk + p * kSliceABytes) = make_uint4(lo[p].x, lo[p].y, hi[p].x, hi[p].y);
   }
   fence_proxy_async_global();
   __syncthreads();
