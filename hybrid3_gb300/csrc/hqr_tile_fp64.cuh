@@ -443,7 +443,7 @@ __device__ __forceinline__ void larfg_newton(double a, double ss, double& tau, d
 }
 
 // Named barriers of the panel loop (0: __syncthreads, 1: the split engine's slicers).
-constexpr int kBarColumn = 2, kBarStep = 3, kBarScalars = 4, kBarSpecial = 5;
+constexpr int kBarColumn = 2, kBarStep = 3, kBarScalars = 4;
 template <int ID, int N>
 __device__ __forceinline__ void bar_sync() { asm volatile("bar.sync %0, %1;" ::"n"(ID), "n"(N) : "memory"); }
 template <int ID, int N>
@@ -453,11 +453,18 @@ constexpr int kPanelWorkers = kWarps - 2;                                       
 constexpr int kPanelItems = 3;       // columns of one worker taken at a time
 constexpr int kPanelGroups = (kMaxW - 1 + kPanelWorkers * kPanelItems - 1) / (kPanelWorkers * kPanelItems);
 constexpr int kPanelRows = 4;        // rows per lane taken at a time: chunks of 128
-// The largest |element| for which the loop's unscaled dots stay in range
-// (larfg_scalars' plain bound is 1e140, about 2^465): the high word from which
-// on a panel takes the general loop.
+// The range of the loop's columns, as high words: with x_c unscaled, its dots,
+// Gram entries and factors stay in range where no element reaches 2^450 and the
+// other column is not much below 2^-400.  Elements are looked at when the panel
+// is loaded.  A column's size is looked at in its own step only, which covers
+// the steps before: a reflection keeps the norm of the rows it acts on, so
+// rows c.. of column j were in step c at least as large as [alpha; x] is in step
+// j > c.  Panels outside take the general loop.
 __host__ __device__ constexpr unsigned kHiExp(int e) { return (unsigned)(1023 + e) << 20; }   // high word of 2^e
-constexpr unsigned kPanelMaxHi = kHiExp(450);
+constexpr unsigned kPanelMaxHi = kHiExp(450), kColumnMinHi = kHiExp(-400);
+__device__ __forceinline__ unsigned magnitude(double v) {   // the high word of |v|; 0 for zero alone
+  return ((unsigned)__double2hiint(v) & 0x7fffffffu) | (__double2loint(v) != 0 ? 1u : 0u);
+}
 
 // TS: unblocked QR of the triangle-on-square panel [R; A] (R w x w, upper part
 // used; A m x w dense), the per-column loop of CORE_dtsqrt: column c's
@@ -465,42 +472,50 @@ constexpr unsigned kPanelMaxHi = kHiExp(450);
 // semantics, R = A, ldr = lda): on A(c:, c).  On return column c of A (below
 // the diagonal for !TS) holds x_c with v_c = x_c scal[c], tau[c], the w x w
 // upper T (ld w) of the block reflector (dlarft 'F','C'); G is scratch.
-// Every |element| is below 2^450.  spec: w ints of scratch.
+// Every |element| is below 2^450.  wide: w ints of scratch.  Returns false, the
+// panel in an undefined state, at the first column that is below 2^-400 and
+// not zero (the same in every thread).
 //
 // Step c: warp 0 waits for column c (updated first by worker 0), takes its
 // norm and scalars; the workers meanwhile take the dots of x_c with every
 // other column -- those right of c, to be updated, and those left of it, for
 // the Gram entry G(b, c) = v_b . v_c; with the scalars they update their
 // columns; warp 4 forms T's column c during step c + 1 (T(0:c, c) = -tau_c
-// T(0:c, 0:c) G(0:c, c)).  A column whose norm or alpha is outside the plain
-// range (spec) is scaled to v by warp 0 and its dots are taken again.
+// T(0:c, 0:c) G(0:c, c)).
 //
 // Larfg: the reflector's convention (LapackLarfg, or tile_kernel.h's).  nref:
 // reflectors formed (columns from there on are updated only).  GRAM false: no
 // Gram entries and no T.
 struct LapackLarfg {
-  // false: outside the plain range (2^-960 <= ss < 2^960, alpha zero or 2^-465
-  // .. 2^465), read off the high words: an FP64 comparison is an FP64
-  // instruction too
+  // false: alpha and x below 2^-400, read off the high words: an FP64 comparison
+  // is an FP64 instruction too.  ss = 0: H = I.
   __device__ static bool scalars(double a, double ss, double& tau, double& scal, double& beta) {
     const unsigned sh = (unsigned)__double2hiint(ss), ah = (unsigned)__double2hiint(a) & 0x7fffffffu;
     tau = 0.0;
     scal = 1.0;
     beta = a;
-    if (sh >= kHiExp(-960) && sh < kHiExp(960) && ah < kHiExp(465) &&
-        (ah >= kHiExp(-465) || (ah | (unsigned)__double2loint(a)) == 0u)) {
-      larfg_newton(a, ss, tau, scal, beta);
-      return true;
-    }
-    return (sh | (unsigned)__double2loint(ss)) == 0u;   // x = 0: H = I
+    if (sh < kHiExp(-800) && ah < kColumnMinHi) return false;
+    if ((sh | (unsigned)__double2loint(ss)) != 0u) larfg_newton(a, ss, tau, scal, beta);
+    return true;
   }
 };
+// By one warp: whether [alpha; x] is zero, and the column's elements r (n of
+// them, at most 32) above alpha are each zero or at least 2^-400: the column
+// was then zero or large enough in every step, and H = I.
+__device__ __forceinline__ bool zero_column(double alpha, const double* x, int m, const double* r, int n) {
+  const int lane = threadIdx.x & 31;
+  unsigned t = magnitude(alpha);
+  for (int i = lane; i < m; i += 32) t |= magnitude(x[i]);
+  if (lane < n && magnitude(r[lane]) < kColumnMinHi) t |= magnitude(r[lane]);
+  return __reduce_or_sync(0xffffffffu, t) == 0u;
+}
 template <bool TS, class Larfg = LapackLarfg, bool GRAM = true>
-__device__ __forceinline__ void panel_qr(double* R, int ldr, double* A, int lda, int m, int w, int nref,
-                                         double* tau, double* scal, int* spec, double* G, double* T) {
+__device__ __forceinline__ bool panel_qr(double* R, int ldr, double* A, int lda, int m, int w, int nref,
+                                         double* tau, double* scal, int* wide, double* G, double* T) {
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   constexpr int kParty = (kPanelWorkers + 1) * 32;                 // the workers and warp 0
   constexpr int kStepParty = (kPanelWorkers + (GRAM ? 1 : 0)) * 32;   // the workers (and warp 4)
+  bool ok = true;
   if (warp == 0) {
     for (int c = 0; c < nref; c++) {
       if (c > 0) bar_sync<kBarColumn, 64>();
@@ -523,29 +538,23 @@ __device__ __forceinline__ void panel_qr(double* R, int ldr, double* A, int lda,
       warp_sums_fixed(ssv);
       const double ss = ssv[0];
       double t, sc, beta;
-      const bool special = !Larfg::scalars(a, ss, t, sc, beta);
+      if (!Larfg::scalars(a, ss, t, sc, beta)) ok = zero_column(a, x + r0, m - r0, R + (size_t)c * ldr, c);
       __syncwarp();
-      if (!special) {
-        if (lane == 0) {
-          tau[c] = t;
-          scal[c] = sc;
-          spec[c] = 0;
-          *al = beta;
-        }
-        __syncwarp();
-        bar_arrive<kBarScalars, kParty>();
-      } else {
-        if (lane == 0) spec[c] = 1;
-        __syncwarp();
-        bar_sync<kBarScalars, kParty>();   // the workers' dots with x are taken
-        if (lane == 0) scal[c] = 1.0;
-        warp_larfg(al, x + r0, m - r0, tau + c);
-        bar_sync<kBarSpecial, kParty>();
+      if (lane == 0) {
+        tau[c] = t;
+        scal[c] = sc;
+        wide[c] = ok ? 0 : 1;
+        *al = beta;
       }
+      __syncwarp();
+      bar_arrive<kBarScalars, kParty>();
+      if (!ok) break;
     }
   } else if (warp == 4) {
     for (int c = 0; GRAM && c < nref; c++) {
       bar_sync<kBarStep, kStepParty>();
+      ok = wide[c] == 0;
+      if (!ok) break;
       double s = 0.0;
       if (lane < c)
         for (int b = 0; b < c; b++) s = fma(lane <= b ? T[lane + b * w] : 0.0, G[b + c * w], s);
@@ -564,36 +573,6 @@ __device__ __forceinline__ void panel_qr(double* R, int ldr, double* A, int lda,
       double acc[kPanelGroups][kPanelItems];
       auto item = [&](int g, int q) { return wi + (g * kPanelItems + q) * kPanelWorkers; };
       auto column = [&](int it) { return it < nupd ? c + 1 + it : it - nupd; };
-      auto dots = [&]() {
-#pragma unroll
-        for (int g = 0; g < kPanelGroups; g++) {
-          if (item(g, 0) >= items) break;
-          const double* aq[kPanelItems];   // (past the last item: column c, the result unused)
-#pragma unroll
-          for (int q = 0; q < kPanelItems; q++) {
-            acc[g][q] = 0.0;
-            aq[q] = A + (size_t)(item(g, q) < items ? column(item(g, q)) : c) * lda;
-          }
-          for (int rb = r0 & ~127; rb < m; rb += 32 * kPanelRows) {
-            double xv[kPanelRows], av[kPanelItems][kPanelRows];
-#pragma unroll
-            for (int i = 0; i < kPanelRows; i++) {
-              const int r = rb + 32 * i + lane;
-              const bool in = r >= r0 && r < m;
-              xv[i] = in ? x[r] : 0.0;
-#pragma unroll
-              for (int q = 0; q < kPanelItems; q++) av[q][i] = in ? aq[q][r] : 0.0;
-            }
-#pragma unroll
-            for (int i = 0; i < kPanelRows; i++)
-              if (rb + 32 * i < m && rb + 32 * i + 31 >= r0)
-#pragma unroll
-                for (int q = 0; q < kPanelItems; q++)
-                  if (q < kPanelItems - 1 || item(g, q) < items) acc[g][q] = fma(xv[i], av[q][i], acc[g][q]);
-          }
-          warp_sums_fixed(acc[g]);
-        }
-      };
       // lane q of a group's first kPanelItems lanes owns item q's scalars
       double rc[kPanelGroups], mul[kPanelGroups];
 #pragma unroll
@@ -603,11 +582,39 @@ __device__ __forceinline__ void panel_qr(double* R, int ldr, double* A, int lda,
         if (it < items && (it < nupd || !TS)) rc[g] = R[c + (size_t)column(it) * ldr];
         if (it < items && it >= nupd) mul[g] = scal[it - nupd];
       }
-      dots();
+#pragma unroll
+      for (int g = 0; g < kPanelGroups; g++) {
+        if (item(g, 0) >= items) break;
+        const double* aq[kPanelItems];   // (past the last item: column c, the result unused)
+#pragma unroll
+        for (int q = 0; q < kPanelItems; q++) {
+          acc[g][q] = 0.0;
+          aq[q] = A + (size_t)(item(g, q) < items ? column(item(g, q)) : c) * lda;
+        }
+        for (int rb = r0 & ~127; rb < m; rb += 32 * kPanelRows) {
+          double xv[kPanelRows], av[kPanelItems][kPanelRows];
+#pragma unroll
+          for (int i = 0; i < kPanelRows; i++) {
+            const int r = rb + 32 * i + lane;
+            const bool in = r >= r0 && r < m;
+            xv[i] = in ? x[r] : 0.0;
+#pragma unroll
+            for (int q = 0; q < kPanelItems; q++) av[q][i] = in ? aq[q][r] : 0.0;
+          }
+#pragma unroll
+          for (int i = 0; i < kPanelRows; i++)
+            if (rb + 32 * i < m && rb + 32 * i + 31 >= r0)
+#pragma unroll
+              for (int q = 0; q < kPanelItems; q++)
+                if (q < kPanelItems - 1 || item(g, q) < items) acc[g][q] = fma(xv[i], av[q][i], acc[g][q]);
+        }
+        warp_sums_fixed(acc[g]);
+      }
       bar_sync<kBarScalars, kParty>();
-      if (spec[c]) {
-        bar_sync<kBarSpecial, kParty>();
-        dots();
+      ok = wide[c] == 0;
+      if (!ok) {
+        bar_sync<kBarStep, kStepParty>();   // warp 4 looks at wide[c] too
+        break;
       }
       const double t = tau[c], sc = scal[c];
       const bool moves = __double_as_longlong(t) != 0;
@@ -661,6 +668,7 @@ __device__ __forceinline__ void panel_qr(double* R, int ldr, double* A, int lda,
     }
   }
   __syncthreads();
+  return ok;
 }
 
 // ---------------------------------------------------------------------------
@@ -855,7 +863,8 @@ __device__ __forceinline__ unsigned load_panel(double* s, int lds, const double*
   return top;
 }
 // The general FP64 column loops (panels with elements of 2^450 and above,
-// infinities or NaN), their T, and scal = 1: their columns are v itself.
+// infinities or NaN, or columns below 2^-400), their T, and scal = 1: their
+// columns are v itself.
 template <bool TS>
 __device__ __noinline__ void panel_qr_general(double* R, int ldr, double* A, int lda, int m, int w, double* tau,
                                               double* scal, double* G, double* T) {
@@ -886,18 +895,21 @@ __device__ void task_geqrt_blk(double* A, double* T, double* tau_g, const TileSh
   {
     const int i0 = b * w;
     const int m = NB - i0;
-    int* spec = reinterpret_cast<int*>(sm + sp.off_red);
-    unsigned* s_top = reinterpret_cast<unsigned*>(spec + kMaxW);
+    int* wide = reinterpret_cast<int*>(sm + sp.off_red);
+    unsigned* s_top = reinterpret_cast<unsigned*>(wide + kMaxW);
     if (kFp64 && threadIdx.x == 0) *s_top = 0u;
     __syncthreads();
     if constexpr (kFp64) {
       double* scal = sm + sp.off_scal;
       note_top(load_panel(sP, NB, A + i0 + (size_t)i0 * NB, NB, m, w), s_top);
       __syncthreads();
-      if (*s_top < kPanelMaxHi)
-        panel_qr<false>(sP, NB, sP, NB, m, w, w, sTau, scal, spec, sG, sTb);
-      else
-        panel_qr_general<false>(sP, NB, sP, NB, m, w, sTau, scal, sG, sTb);
+      bool general = *s_top >= kPanelMaxHi;
+      if (!general && !panel_qr<false>(sP, NB, sP, NB, m, w, w, sTau, scal, wide, sG, sTb)) {
+        general = true;
+        load_panel(sP, NB, A + i0 + (size_t)i0 * NB, NB, m, w);
+        __syncthreads();
+      }
+      if (general) panel_qr_general<false>(sP, NB, sP, NB, m, w, sTau, scal, sG, sTb);
       // R and V = x scal to the tile; V also to the trailing update's buffers
       resident = m - w <= sh.RC;
       double* sVb = sm + sp.off_vb;
@@ -964,20 +976,26 @@ __device__ void task_tsqrt_blk(double* A1, double* A2, double* T, double* tau_g,
   bool resident = false;   // V and T left in shared memory for the trailing update
   {
     const int i0 = b * w;
-    int* spec = reinterpret_cast<int*>(sm + sp.off_red);
-    unsigned* s_top = reinterpret_cast<unsigned*>(spec + kMaxW);
+    int* wide = reinterpret_cast<int*>(sm + sp.off_red);
+    unsigned* s_top = reinterpret_cast<unsigned*>(wide + kMaxW);
     if (kFp64 && threadIdx.x == 0) *s_top = 0u;
     __syncthreads();
     if constexpr (kFp64) {
       double* scal = sm + sp.off_scal;
-      const unsigned top = load_panel(sA, NB, A2 + (size_t)i0 * NB, NB, NB, w, a2_upper ? i0 : -1);
       // R's strictly lower part (the GEQRT's V) is neither used nor counted
-      note_top(max(top, load_panel(sR, w, A1 + i0 + (size_t)i0 * NB, NB, w, w, 0)), s_top);
+      auto load = [&]() {
+        const unsigned top = load_panel(sA, NB, A2 + (size_t)i0 * NB, NB, NB, w, a2_upper ? i0 : -1);
+        return max(top, load_panel(sR, w, A1 + i0 + (size_t)i0 * NB, NB, w, w, 0));
+      };
+      note_top(load(), s_top);
       __syncthreads();
-      if (*s_top < kPanelMaxHi)
-        panel_qr<true>(sR, w, sA, NB, NB, w, w, sTau, scal, spec, sG, sTb);
-      else
-        panel_qr_general<true>(sR, w, sA, NB, NB, w, sTau, scal, sG, sTb);
+      bool general = *s_top >= kPanelMaxHi;
+      if (!general && !panel_qr<true>(sR, w, sA, NB, NB, w, w, sTau, scal, wide, sG, sTb)) {
+        general = true;
+        load();
+        __syncthreads();
+      }
+      if (general) panel_qr_general<true>(sR, w, sA, NB, NB, w, sTau, scal, sG, sTb);
       // V = x scal to the tile (a merge: its upper triangle) and to the
       // trailing update's buffer
       resident = NB <= sh.RC;

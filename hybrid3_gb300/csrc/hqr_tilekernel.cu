@@ -73,7 +73,7 @@ __global__ void __launch_bounds__(kThreads) k_panel(int row, int col, double* A1
   double* sA = sm;
   double* tau = sA + (size_t)row * col;
   double* scal = tau + kMaxW;
-  int* spec = reinterpret_cast<int*>(scal + kMaxW);
+  int* wide = reinterpret_cast<int*>(scal + kMaxW);
   double* sR = scal + kMaxW + kMaxW / 2;
   for (int e = threadIdx.x; e < row * col; e += kThreads) sA[e] = A2[e % row + (size_t)(e / row) * lda2];
   if (TS)
@@ -82,9 +82,9 @@ __global__ void __launch_bounds__(kThreads) k_panel(int row, int col, double* A1
   __syncthreads();
   const int nref = (!TS && row == col) ? col - 1 : col;
   if (TS)
-    panel_qr<true, TileLarfg, false>(sR, col, sA, row, row, col, nref, tau, scal, spec, nullptr, nullptr);
+    panel_qr<true, TileLarfg, false>(sR, col, sA, row, row, col, nref, tau, scal, wide, nullptr, nullptr);
   else
-    panel_qr<false, TileLarfg, false>(sA, row, sA, row, row, col, nref, tau, scal, spec, nullptr, nullptr);
+    panel_qr<false, TileLarfg, false>(sA, row, sA, row, row, col, nref, tau, scal, wide, nullptr, nullptr);
   for (int e = threadIdx.x; e < row * col; e += kThreads) {
     const int r = e % row, c = e / row;
     double v = sA[e];
