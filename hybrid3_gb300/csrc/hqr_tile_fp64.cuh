@@ -483,10 +483,13 @@ __device__ __forceinline__ unsigned magnitude(double v) {   // the high word of 
 // columns; warp 4 forms T's column c during step c + 1 (T(0:c, c) = -tau_c
 // T(0:c, 0:c) G(0:c, c)).
 //
-// Larfg: the reflector's convention (LapackLarfg, or tile_kernel.h's).  nref:
+// Larfg: the reflector's convention (LapackLarfg, or tile_kernel.h's): the two
+// numbers of column c that scalars() puts into tau[c] and scal[c], and update()'s
+// change of a column from its dot with x_c: r_c -= s, a -= f x_c.  nref:
 // reflectors formed (columns from there on are updated only).  GRAM false: no
 // Gram entries and no T.
 struct LapackLarfg {
+  static constexpr bool kSplitFactor = false;
   // false: alpha and x below 2^-400, read off the high words: an FP64 comparison
   // is an FP64 instruction too.  ss = 0: H = I.
   __device__ static bool scalars(double a, double ss, double& tau, double& scal, double& beta) {
@@ -497,6 +500,12 @@ struct LapackLarfg {
     if (sh < kHiExp(-800) && ah < kColumnMinHi) return false;
     if ((sh | (unsigned)__double2loint(ss)) != 0u) larfg_newton(a, ss, tau, scal, beta);
     return true;
+  }
+  __device__ static bool moves(double tau) { return __double_as_longlong(tau) != 0; }   // (tau = 0 is +0)
+  // d = x . a, t: tau (of a Gram entry: the other column's scal).  v = x scal
+  __device__ static void update(double& d, double r, double t, double scal, double& s, double& f) {
+    s = fma(scal, d, r) * t;
+    f = s * scal;
   }
 };
 // By one warp: whether [alpha; x] is zero, and the column's elements r (n of
@@ -617,7 +626,7 @@ __device__ __forceinline__ bool panel_qr(double* R, int ldr, double* A, int lda,
         break;
       }
       const double t = tau[c], sc = scal[c];
-      const bool moves = __double_as_longlong(t) != 0;
+      const bool moves = Larfg::moves(t);
 #pragma unroll
       for (int g = 0; g < kPanelGroups; g++) {
         if (item(g, 0) >= items) break;
@@ -626,8 +635,8 @@ __device__ __forceinline__ bool panel_qr(double* R, int ldr, double* A, int lda,
 #pragma unroll
         for (int q = 1; q < kPanelItems; q++) d = lane == q ? acc[g][q] : d;
         // update: s = tau (v_c . a_j + r_cj); Gram: G(b, c) = v_b . v_c
-        const double s = fma(sc, d, rc[g]) * (mine < nupd ? t : mul[g]);
-        const double f = s * sc;
+        double s, f;
+        Larfg::update(d, rc[g], mine < nupd ? t : mul[g], sc, s, f);
         if (lane < kPanelItems && mine < items) {
           if (mine < nupd)
             R[c + (size_t)(c + 1 + mine) * ldr] = rc[g] - s;
@@ -640,7 +649,15 @@ __device__ __forceinline__ bool panel_qr(double* R, int ldr, double* A, int lda,
           if (it >= nupd) break;
           const double fq = __shfl_sync(0xffffffffu, f, q);
           double* aj = A + (size_t)(c + 1 + it) * lda;
-          for (int rb = r0 & ~127; rb < m && moves; rb += 32 * kPanelRows) {
+          bool whole = moves;   // a -= f x with f as one factor
+          if (Larfg::kSplitFactor) {
+            // (a factor that is not in range is two: a -= (t x) d)
+            const unsigned fh = (unsigned)__double2hiint(fq) & 0x7fffffffu;
+            whole = fh >= kHiExp(-960) && fh < kHiExp(960);
+            const double dq = __shfl_sync(0xffffffffu, d, q);
+            for (int r = r0 + lane; r < m && !whole; r += 32) aj[r] = fma(-(t * x[r]), dq, aj[r]);
+          }
+          for (int rb = r0 & ~127; rb < m && whole; rb += 32 * kPanelRows) {
             double xv[kPanelRows], av[kPanelRows];
 #pragma unroll
             for (int i = 0; i < kPanelRows; i++) {

@@ -39,21 +39,32 @@ namespace tk {
 // ---------------------------------------------------------------------------
 
 // The reflector of this file's kernels: beta = +sqrt(a^2 + ss), head = a -
-// beta, v = x / head, tau = 2 head^2 / (head^2 + ss); no guard (x = 0 and a > 0
-// divides by zero, as the reference does).
+// beta, v = x / head, tau = t head^2 with t = 2 / (head^2 + ss); no guard (x = 0
+// and a > 0 divides by zero, as the reference does).  The loop works with t and
+// head (in tau[c] and scal[c]) on x as it is: where x is so small that head is
+// zero, v is infinite but t, and with it R and the other columns, is not.
 struct TileLarfg {
-  __device__ static bool scalars(double a, double ss, double& tau, double& scal, double& beta) {
+  static constexpr bool kSplitFactor = true;
+  __device__ static bool scalars(double a, double ss, double& t, double& head, double& beta) {
     beta = sqrt(ss + a * a);
-    const double head = a - beta;
-    scal = 1.0 / head;
-    tau = 2.0 / (head * head + ss) * head * head;
+    head = a - beta;
+    t = 2.0 / (head * head + ss);
     return true;
+  }
+  __device__ static bool moves(double) { return true; }
+  __device__ static void update(double& d, double r, double t, double head, double& s, double& f) {
+    d = fma(head, r, d);
+    s = t * head * d;
+    f = t * d;
   }
 };
 
 // Doubles of shared memory of k_panel beyond its row x col panel.
 constexpr int kPanelExtra = 2 * kMaxW + kMaxW / 2 + kMaxW * kMaxW;
 constexpr size_t kPanelSmem = 220 * 1024;
+// k_panel's copy of a panel for its application: its row x col columns, then
+// kMaxW t and kMaxW heads.
+constexpr size_t kPanelCopy = kPanelSmem / 8 + 2 * kMaxW;
 // The widest panel (at most kMaxW columns) of `row` rows that fits (0: none).
 int panel_cols(int row) {
   const long fit = ((long)kPanelSmem / 8 - kPanelExtra) / (row > 0 ? row : 1);
@@ -64,11 +75,13 @@ int panel_cols(int row) {
 // tile_sub_dtsqr2 on [A1 (upper col x col); A2], A2 becomes V.  !TS:
 // tile_sub_dgeqr2 on A2 (row x col) alone, V also to Y (ld lda, unit
 // diagonal); a square panel has no last reflector (TAU(col-1) is left as it
-// is and Y(col-1, col-1) = 0).  The loop's FP64 work (4 row col^2 flops on one
-// SM) and its chain of col norms bound it.
+// is and Y(col-1, col-1) = 0).  X (or null): kPanelCopy doubles that receive the
+// reflectors as [head; x] (ld row; !TS: head on the diagonal), t and head, from
+// which H = I - t [head; x] [head; x]^T needs no division by head.  The loop's
+// FP64 work (4 row col^2 flops on one SM) and its chain of col norms bound it.
 template <bool TS>
 __global__ void __launch_bounds__(kThreads) k_panel(int row, int col, double* A1, int lda1, double* A2, int lda2,
-                                                    double* TAU, double* Y) {
+                                                    double* TAU, double* Y, double* X) {
   extern __shared__ double sm[];
   double* sA = sm;
   double* tau = sA + (size_t)row * col;
@@ -85,6 +98,20 @@ __global__ void __launch_bounds__(kThreads) k_panel(int row, int col, double* A1
     panel_qr<true, TileLarfg, false>(sR, col, sA, row, row, col, nref, tau, scal, wide, nullptr, nullptr);
   else
     panel_qr<false, TileLarfg, false>(sA, row, sA, row, row, col, nref, tau, scal, wide, nullptr, nullptr);
+  if (X) {
+    for (int e = threadIdx.x; e < row * col; e += kThreads) X[e] = !TS && e % row == e / row ? scal[e / row] : sA[e];
+    for (int c = threadIdx.x; c < col; c += kThreads) {
+      X[(size_t)row * col + c] = tau[c];
+      X[(size_t)row * col + kMaxW + c] = scal[c];
+    }
+    __syncthreads();
+  }
+  for (int c = threadIdx.x; c < nref; c += kThreads) {
+    const double head = scal[c];
+    TAU[c] = tau[c] * head * head;
+    scal[c] = 1.0 / head;
+  }
+  __syncthreads();
   for (int e = threadIdx.x; e < row * col; e += kThreads) {
     const int r = e % row, c = e / row;
     double v = sA[e];
@@ -95,7 +122,6 @@ __global__ void __launch_bounds__(kThreads) k_panel(int row, int col, double* A1
   if (TS)
     for (int e = threadIdx.x; e < col * col; e += kThreads)
       if (e % col <= e / col) A1[e % col + (size_t)(e / col) * lda1] = sR[e];
-  for (int c = threadIdx.x; c < nref; c += kThreads) TAU[c] = tau[c];
 }
 
 // out[c] = sum_{r < n} x[r] * (base + c*ld)[r] for c < nc: one warp per column.
@@ -362,10 +388,10 @@ __global__ void __launch_bounds__(kThreads) k_dlarft_block(int row, int col, int
   }
 }
 
-// One column of W = Y^T a: out[r] = [first[r] +] sum_{q >= (lower ? r : 0)}
-// Y(q, r) a(q), r < Y_col, by the CTA: a warp takes four r at a time.
+// One column of W = Y^T a: out[r] = [first[r] (head[r] first[r]) +] sum_{q >=
+// (lower ? r : 0)} Y(q, r) a(q), r < Y_col, by the CTA: a warp takes four r at a time.
 __device__ void column_yta(int row, int Y_col, const double* Y, int ldy, const double* a, const double* first,
-                           double* out, bool lower) {
+                           double* out, bool lower, const double* head = nullptr) {
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   for (int r0 = 4 * warp; r0 < Y_col; r0 += 4 * kWarps) {
     double s[4] = {0.0, 0.0, 0.0, 0.0};
@@ -378,7 +404,10 @@ __device__ void column_yta(int row, int Y_col, const double* Y, int ldy, const d
     warp_sums_fixed(s);
 #pragma unroll
     for (int p = 0; p < 4; p++)
-      if (r0 + p < Y_col && lane == p) out[r0 + p] = (first ? first[r0 + p] : 0.0) + s[p];
+      if (r0 + p < Y_col && lane == p) {
+        const double top = first ? first[r0 + p] : 0.0;
+        out[r0 + p] = (head ? head[r0 + p] * top : top) + s[p];
+      }
   }
   __syncthreads();
 }
@@ -448,12 +477,14 @@ __global__ void __launch_bounds__(kThreads) k_sub_dlarfb(int row, int Y_col, int
 //   part 0: the whole update; 1: tile_dssrfb_head (A1 update, D kept in U,
 //   ld over_row); 2: tile_dssrfb_tail (A2 -= Y D from U).
 // Quirk kept: rows Y_col..over_row-1 of A1 are zeroed (A1 -= its own copy).
-// transT: T read transposed (tile_return_dssrfb).  D: over_row x A_col, D2:
-// Y_col x A_col global scratch.  Columns as in k_sub_dlarfb.
+// transT: T read transposed (tile_return_dssrfb).  head (or null, for 1): what
+// Y has above A2's rows, one number a column (over_row = Y_col).  D: over_row x
+// A_col, D2: Y_col x A_col global scratch.  Columns as in k_sub_dlarfb.
 __global__ void __launch_bounds__(kThreads) k_sub_dssrfb(int over_row, int under_row, int Y_col, int A_col,
                                                           const double* Y, int ldy, const double* T, int ldt,
                                                           double* A1, int lda1, double* A2, int lda2, double* D,
-                                                          double* D2, double* U, int part, int transT) {
+                                                          double* D2, double* U, int part, int transT,
+                                                          const double* head) {
   __shared__ double sums[kThreads];
   for (int c = blockIdx.x; c < A_col; c += gridDim.x) {
     double* a1 = A1 + (size_t)c * lda1;
@@ -462,11 +493,11 @@ __global__ void __launch_bounds__(kThreads) k_sub_dssrfb(int over_row, int under
     if (part != 2) {
       double* d = D + (size_t)c * over_row;
       double* d2 = D2 + (size_t)c * Y_col;
-      column_yta(under_row, min(Y_col, over_row), Y, ldy, a2, a1, d, false);
+      column_yta(under_row, min(Y_col, over_row), Y, ldy, a2, a1, d, false, head);
       column_tw(Y_col, T, ldt, transT, d, d2, sums);
       for (int r = threadIdx.x; r < over_row; r += kThreads) {
         const double v = r < Y_col ? d2[r] : a1[r];
-        a1[r] -= v;
+        a1[r] -= head ? head[r] * v : v;
         if (part == 1) U[r + (size_t)c * over_row] = v;
       }
       if (part == 1) continue;
@@ -631,19 +662,24 @@ void sub_dlarfb(cudaStream_t s, int row, int Y_col, int A_col, const double* Y, 
 }
 void sub_dssrfb(cudaStream_t s, int over_row, int under_row, int Y_col, int A_col, const double* Y, int ldy,
                 const double* T, int ldt, double* A1, int lda1, double* A2, int lda2, double* D, double* D2,
-                double* U, int part, int transT) {
+                double* U, int part, int transT, const double* head = nullptr) {
   k_sub_dssrfb<<<column_blocks(A_col), kThreads, 0, s>>>(over_row, under_row, Y_col, A_col, Y, ldy, T, ldt, A1, lda1,
-                                                        A2, lda2, D, D2, U, part, transT);
+                                                        A2, lda2, D, D2, U, part, transT, head);
 }
 // Scratch of the panels wider than one column loop: T and G of a loop's
-// columns, and D, D2 of their application to the rest.
-size_t panel_scratch(int col) { return 2 * (size_t)kMaxW * kMaxW + 2 * (size_t)kMaxW * col; }
+// columns, D, D2 of their application to the rest, and their copy.
+struct PanelScratch {
+  double *T, *G, *D, *D2, *X;
+  PanelScratch(double* base, int col) : T(base), G(T + kMaxW * kMaxW), D(G + kMaxW * kMaxW), D2(D + (size_t)kMaxW * col),
+                                        X(D2 + (size_t)kMaxW * col) {}
+  static size_t size(int col) { return 2 * (size_t)kMaxW * kMaxW + 2 * (size_t)kMaxW * col + kPanelCopy; }
+};
 
 // tile_sub_dgeqr2: panels of at most kMaxW columns in shared memory, each
 // applied to the columns right of it; taller ones than fit go column by
 // column through global memory (k_sub_dgeqr2).
 void sub_dgeqr2(cudaStream_t s, int row, int col, double* A, int lda, double* TAU, double* Y, double* work) {
-  double *T = work, *G = T + kMaxW * kMaxW, *D = G + kMaxW * kMaxW, *D2 = D + (size_t)kMaxW * col;
+  const PanelScratch w(work, col);
   const int cw = panel_cols(row);
   if (cw < 1) {
     k_sub_dgeqr2<<<1, kThreads, (size_t)col * sizeof(double), s>>>(row, col, A, lda, TAU, Y);
@@ -654,17 +690,17 @@ void sub_dgeqr2(cudaStream_t s, int row, int col, double* A, int lda, double* TA
     const int jb = col - j < cw ? col - j : cw, rows = row - j, rest = col - j - jb;
     double* Aj = A + j + (size_t)j * lda;
     double* Yj = Y + j + (size_t)j * lda;
-    k_panel<false><<<1, kThreads, ((size_t)rows * jb + kPanelExtra) * sizeof(double), s>>>(rows, jb, nullptr, 0, Aj,
-                                                                                          lda, TAU + j, Yj);
+    k_panel<false><<<1, kThreads, ((size_t)rows * jb + kPanelExtra) * sizeof(double), s>>>(
+        rows, jb, nullptr, 0, Aj, lda, TAU + j, Yj, rest > 0 ? w.X : nullptr);
     if (rest == 0) break;
-    sub_dlarft(s, rows, jb, Yj, lda, TAU + j, T, kMaxW, G, true, true);
-    sub_dlarfb(s, rows, jb, rest, Yj, lda, T, kMaxW, Aj + (size_t)jb * lda, lda, D, D2, 0, true);
+    sub_dlarft(s, rows, jb, w.X, rows, w.X + (size_t)rows * jb, w.T, kMaxW, w.G, true, true);
+    sub_dlarfb(s, rows, jb, rest, w.X, rows, w.T, kMaxW, Aj + (size_t)jb * lda, lda, w.D, w.D2, 0, true);
   }
 }
 // tile_sub_dtsqr2, in the same way.
 void sub_dtsqr2(cudaStream_t s, int row, int col, double* A1, int lda1, double* A2, int lda2, double* TAU,
                 double* work) {
-  double *T = work, *G = T + kMaxW * kMaxW, *D = G + kMaxW * kMaxW, *D2 = D + (size_t)kMaxW * col;
+  const PanelScratch w(work, col);
   const int cw = panel_cols(row);
   if (cw < 1) {
     k_sub_dtsqr2<<<1, kThreads, (size_t)col * sizeof(double), s>>>(row, col, A1, lda1, A2, lda2, TAU);
@@ -675,12 +711,13 @@ void sub_dtsqr2(cudaStream_t s, int row, int col, double* A1, int lda1, double* 
     const int jb = col - j < cw ? col - j : cw, rest = col - j - jb;
     double* A1j = A1 + j + (size_t)j * lda1;
     double* A2j = A2 + (size_t)j * lda2;
-    k_panel<true><<<1, kThreads, ((size_t)row * jb + kPanelExtra) * sizeof(double), s>>>(row, jb, A1j, lda1, A2j,
-                                                                                        lda2, TAU + j, nullptr);
+    k_panel<true><<<1, kThreads, ((size_t)row * jb + kPanelExtra) * sizeof(double), s>>>(
+        row, jb, A1j, lda1, A2j, lda2, TAU + j, nullptr, rest > 0 ? w.X : nullptr);
     if (rest == 0) break;
-    sub_dlarft(s, row, jb, A2j, lda2, TAU + j, T, kMaxW, G, false, true);
-    sub_dssrfb(s, jb, row, jb, rest, A2j, lda2, T, kMaxW, A1j + (size_t)jb * lda1, lda1, A2j + (size_t)jb * lda2,
-               lda2, D, D2, nullptr, 0, 0);
+    const double *t = w.X + (size_t)row * jb, *head = t + kMaxW;
+    sub_dlarft(s, row, jb, w.X, row, t, w.T, kMaxW, w.G, false, true);
+    sub_dssrfb(s, jb, row, jb, rest, w.X, row, w.T, kMaxW, A1j + (size_t)jb * lda1, lda1, A2j + (size_t)jb * lda2,
+               lda2, w.D, w.D2, nullptr, 0, 0, head);
   }
 }
 
@@ -711,7 +748,7 @@ void tile_sub_dgeqr2(const int row, const int col, double* A, const int lda, dou
   double* dA = call.arg(A, extent(lda, row, col), true);
   double* dT = call.arg(TAU, col, true);
   double* dY = call.arg(Y, extent(lda, row, col), true);
-  const size_t w = call.scratch(hqr::tk::panel_scratch(col));
+  const size_t w = call.scratch(hqr::tk::PanelScratch::size(col));
   double* base = call.bind();
   if (!base) return;
   hqr::tk::sub_dgeqr2(call.stream(), row, col, call.view(A, dA), lda, call.view(TAU, dT), call.view(Y, dY), base + w);
@@ -727,7 +764,7 @@ void tile_sub_dtsqr2(const int row, const int col, double* A1, const int lda1, d
   double* d1 = call.arg(A1, extent(lda1, col, col), true);
   double* d2 = call.arg(A2, extent(lda2, row, col), true);
   double* dt = call.arg(TAU, col, true);
-  const size_t w = call.scratch(hqr::tk::panel_scratch(col));
+  const size_t w = call.scratch(hqr::tk::PanelScratch::size(col));
   double* base = call.bind();
   if (!base) return;
   hqr::tk::sub_dtsqr2(call.stream(), row, col, call.view(A1, d1), lda1, call.view(A2, d2), lda2,
@@ -804,7 +841,7 @@ void tile_dgeqrt(const int row, const int col, const int block, double* A, const
   double* dT = call.arg(T, extent(ldt, col, col), true);
   const size_t g = call.scratch((size_t)col * col);
   const size_t d = call.scratch((size_t)row * col), d2 = call.scratch((size_t)row * col);
-  const size_t w = call.scratch(hqr::tk::panel_scratch(col));
+  const size_t w = call.scratch(hqr::tk::PanelScratch::size(col));
   double* base = call.bind();
   if (!base) return;
   A = call.view(A, dA);
@@ -836,7 +873,7 @@ void tile_dtsqrt(const int row, const int col, const int block, double* A1, cons
   double* dT = call.arg(T, extent(ldt, col, col), true);
   const size_t g = call.scratch((size_t)col * col);
   const size_t d = call.scratch((size_t)block * col), dd = call.scratch((size_t)block * col);
-  const size_t w = call.scratch(hqr::tk::panel_scratch(col));
+  const size_t w = call.scratch(hqr::tk::PanelScratch::size(col));
   double* base = call.bind();
   if (!base) return;
   A1 = call.view(A1, d1);
