@@ -310,7 +310,10 @@ __global__ void k_trsmt_step(const double* __restrict__ RA, int MT, int NB, doub
 // 32 x 32 diagonal block in registers, divided by the diagonal (one shuffle and
 // one FMA a row instead of a barrier, a product and an FMA), and the blocks
 // beside it are loaded while the warp before it solves.  N = 8192, 16
-// right-hand sides: 64 steps of 27 us, 87 us before.
+// right-hand sides: 64 steps of 27 us, 87 us before.  A block with an element
+// R_rj / R_jj that is not well inside the FP64 range (or a reciprocal that is
+// not) is held as it is: y_j = v_j / R_jj, then v_r -= R_rj y_j, a product more
+// a row, as k_trsm_step does.
 constexpr int kTriMaxNB = 256;
 template <bool TRANS>
 __global__ void __launch_bounds__(kTriMaxNB) k_tri_step(const double* __restrict__ RA, int MT, int NB, double* __restrict__ C, int i, int NT) {
@@ -328,13 +331,27 @@ __global__ void __launch_bounds__(kTriMaxNB) k_tri_step(const double* __restrict
   const double* Rkk = RA + ((long)k + (long)k * MT) * tile;
   // element (r, 32 bb + j) of the triangular factor
   auto at = [&](int bb, int j) { return TRANS ? Rkk[32 * bb + j + (long)r * NB] : Rkk[r + (long)(32 * bb + j) * NB]; };
+  // 2^-900 <= |v| < 2^900, read off the high word
+  auto in_range = [](double v) {
+    return ((unsigned)__double2hiint(v) & 0x7fffffffu) - ((1023u - 900u) << 20) < (1800u << 20);
+  };
   double rs[32], inv = 0.0;
+  bool plain = true;
   if (diag) {
     inv = 1.0 / Rkk[r + (long)r * NB];
 #pragma unroll
     for (int j = 0; j < 32; j++) rs[j] = (TRANS ? j < lane : j > lane) ? at(b, j) : 0.0;
 #pragma unroll
-    for (int j = 0; j < 32; j++) rs[j] *= __shfl_sync(full, inv, j);
+    for (int j = 0; j < 32; j++) {
+      const bool zero = (__double2hiint(rs[j]) << 1 | __double2loint(rs[j])) == 0;
+      rs[j] *= __shfl_sync(full, inv, j);
+      plain = plain && (zero || in_range(rs[j]));
+    }
+    plain = __all_sync(full, plain && in_range(inv));
+    if (!plain) {
+#pragma unroll
+      for (int j = 0; j < 32; j++) rs[j] = (TRANS ? j < lane : j > lane) ? at(b, j) : 0.0;
+    }
   }
   double v = Ck[r];
   if (!first) {
@@ -383,13 +400,23 @@ __global__ void __launch_bounds__(kTriMaxNB) k_tri_step(const double* __restrict
       for (int j = 0; j < 32; j++) pf[j] = at(bb, j);
     }
     if (b == bb) {
+      if (plain) {
 #pragma unroll
-      for (int jj = 0; jj < 32; jj++) {
-        const int j = TRANS ? jj : 31 - jj;
-        const double y = __shfl_sync(full, v, j);
-        if (TRANS ? lane > j : lane < j) v = fma(-rs[j], y, v);
+        for (int jj = 0; jj < 32; jj++) {
+          const int j = TRANS ? jj : 31 - jj;
+          const double y = __shfl_sync(full, v, j);
+          if (TRANS ? lane > j : lane < j) v = fma(-rs[j], y, v);
+        }
+        v *= inv;
+      } else {
+#pragma unroll
+        for (int jj = 0; jj < 32; jj++) {
+          const int j = TRANS ? jj : 31 - jj;
+          const double y = __shfl_sync(full, v * inv, j);
+          if (lane == j) v = y;
+          if (TRANS ? lane > j : lane < j) v = fma(-rs[j], y, v);
+        }
       }
-      v *= inv;
       sy[r] = v;
     }
     __syncthreads();
