@@ -245,7 +245,7 @@ static int update_columns(const Geometry& g, long long tiles, long long path, in
 static void set_columns(DagParams& p, const Geometry& g, int cb, int cols) {
   p.sh = shape_of(g);
   if (p.oz) return;
-  p.sh.CB = cb;
+  p.ucols = cb;
   p.NC = (cols + cb - 1) / cb;
   p.count_every = g.CB / cb;
 }
