@@ -110,7 +110,8 @@ int dag_sm_count() {
   return v;
 }
 
-// The largest dynamic shared memory a kernel has been opted in to, per device.
+// The largest dynamic shared memory a kernel has been opted in to, per device
+// (one record a kernel: a smaller opt-in would take a larger one back).
 struct SmemOptIn {
   std::mutex mu;
   size_t bytes[kCacheDevices] = {};
@@ -695,19 +696,10 @@ int launch_factor_external(const Geometry& g, const ExternalScratch& x, double* 
   p.ctl = x.ctl;
   p.stats = x.stats;
   p.timeout_ns = timeout_ns;
-  static SmemOptIn opted;
-  {
-    const cudaError_t e = opt_in(opted, dag_exec_kernel<false>, g.smem_bytes);
-    if (e != cudaSuccess) return record_cuda_error(e, "cudaFuncSetAttribute(dag_exec_kernel)");
-  }
   const int blocks = (p.n_ids + 255) / 256;
   dag_init_kernel<<<blocks, 256, 0, stream>>>(p);
   dag_seed_kernel<<<blocks, 256, 0, stream>>>(p);
-  const int grid = std::min(dag_sm_count(), std::max(1, p.n_tasks));
-  dag_exec_kernel<false><<<grid, kThreads, g.smem_bytes, stream>>>(p);
-  cudaError_t e = cudaGetLastError();
-  if (e != cudaSuccess) return record_cuda_error(e, "dag_exec_kernel launch");
-  return HQR_OK;
+  return launch_exec<false>(p, g, stream);
 }
 
 int external_status(const ExternalScratch& x, cudaStream_t stream) {
