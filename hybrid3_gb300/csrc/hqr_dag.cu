@@ -154,10 +154,11 @@ static int launch_exec(const DagParams& p, const Geometry& g, cudaStream_t strea
   return HQR_OK;
 }
 
-static int run_dag(DagParams& p, DagWorkspace* ws, const Geometry& g, cudaStream_t stream) {
+// reserve: ids to reserve the scheduler's tables for, at least this run's.
+static int run_dag(DagParams& p, DagWorkspace* ws, const Geometry& g, cudaStream_t stream, long long reserve = 0) {
   p.sp = SmemPlan::make(p.sh);
   p.n_ids = id_end(p);
-  int rc = dag_workspace_reserve(ws, (size_t)p.n_ids);
+  int rc = dag_workspace_reserve(ws, (size_t)std::max((long long)p.n_ids, reserve));
   if (rc != HQR_OK) return rc;
   p.cnt = ws->cnt;
   p.qhi = ws->qhi;
@@ -307,6 +308,29 @@ static void set_oz(DagParams& p, const Geometry& g, const OzWorkspace* oz, int c
   }
 }
 
+// The most task ids that Q generation or an application to up to NT tile columns
+// takes on the plan of factorization f (`chain` tasks down a column).  The
+// factorization reserves the scheduler's tables for them as well: a later call
+// on the plan then allocates nothing, so that it can be captured into a graph,
+// keeps the addresses that an earlier graph holds, and loses no status that has
+// not been read yet.  Their tasks can be narrower than the factorization's.
+static long long plan_apply_ids(const DagParams& f, const Geometry& g, int chain) {
+  long long below = 0, q_tiles = 0;   // tiles of one column; of Q generation
+  for (int i = 0; i < g.steps; i++) {
+    below += g.MT - i;
+    q_tiles += (long long)(g.NT - i) * (g.MT - i);
+  }
+  const long long path = chain + g.steps;
+  auto ids = [&](long long tiles, int CT) {
+    long long nc = f.oz ? g.NB / oz::kN / oz_chunks(tiles, path) : g.NB / update_columns(g, tiles, path, g.NB);
+    if (!f.oz && CT == 1) nc = g.NB / 8;   // (few right-hand sides in one tile column: any width)
+    return g.steps * ((long long)g.MT + f.dmax + ((long long)g.MT + f.dmax) * CT * nc);
+  };
+  long long most = g.M == g.N ? ids(q_tiles, g.NT) : 0;
+  for (int CT = 1; CT <= g.NT; CT++) most = std::max(most, ids(CT * below, CT));
+  return most;
+}
+
 // Domains and merge storage of a domain tree (tw null or tw->S == 0: flat).
 static void set_tree(DagParams& p, const Geometry& g, const TreeWorkspace* tw) {
   if (!tw || tw->S <= 0 || tw->S >= g.MT) {
@@ -368,7 +392,7 @@ int launch_factor(const Geometry& g, DagWorkspace* ws, double* dA, double* dT, d
     n += m * (p.nblk + (p.prep ? 1 : 0)) + m * p.NC * (g.NT - 1 - i);
   }
   p.n_tasks = (int)n;
-  return run_dag(p, ws, g, stream);
+  return run_dag(p, ws, g, stream, plan_apply_ids(p, g, chain));
 }
 
 int launch_apply_qt(const Geometry& g, DagWorkspace* ws, const double* dA, double* dT,
