@@ -186,9 +186,11 @@ static int run_dag(DagParams& p, DagWorkspace* ws, const Geometry& g, cudaStream
 // the shorter chain gains.  Measured, against whole panel blocks: FP64 n =
 // 2048, NB 256: factorization 73 -> 38 ms; n = 4096: 155 -> 118 ms; split n =
 // 3072 (against blocks that released their dependents in phases): QR + Q 35.7
-// -> 28.4 ms; split n = 16384 unchanged.  FP32 panels have no such steps: their
-// blocks take half the time and are latency, not work (32768 x 8192: 355 ms
-// with none, 356 from 300 tiles on, 382 from 6000).
+// -> 28.4 ms; split n = 16384 unchanged.  With FP32 panels only the last step is
+// one (no tiles left): their blocks take half the time and are latency, not work
+// (factorization, ms, none / the last step: 4 x 4 tiles 3.46 / 3.39, 16 x 16
+// 14.7 / 14.6, 256 x 64 292 / 295, 1000 x 2 103.1 / 104.5; 32768 x 8192 then:
+// 355 / - , 356 from 300 tiles on, 382 from 6000).
 //
 // Such a task takes a part of a block's w columns: the chain through a tile is
 // its panel blocks and the first part after each, and a part of 8 / 16 / 32
