@@ -10,15 +10,25 @@
 namespace hqr {
 
 // Task ids of the plain FP64 factorization with nc column blocks per update
-// tile and no trailing-update tasks, and the bytes of scratch that
-// hqr_geqrf_noalloc carves for n_ids ids.
+// tile and no trailing-update tasks, and the scratch that hqr_geqrf_noalloc
+// carves for n_ids ids.
 static size_t coarse_task_ids(const Geometry& g, int nc) {
   return (size_t)g.steps * g.MT * (g.NB / g.w) + (size_t)g.steps * g.NT * g.MT * nc;
 }
-size_t external_bytes(const Geometry& g, size_t n_ids) {
-  auto round256 = [](size_t b) { return (b + 255) & ~size_t(255); };
-  return round256((size_t)g.M * g.N * sizeof(double)) + 3 * round256(n_ids * sizeof(int)) +
-         round256(kExternalCtlBytes) + round256(kExternalStatsBytes);
+ExternalLayout external_layout(const Geometry& g, size_t n_ids) {
+  ExternalLayout l{};
+  auto carve = [&](size_t b) {
+    const size_t at = l.bytes;
+    l.bytes += (b + 255) & ~size_t(255);
+    return at;
+  };
+  l.T = carve((size_t)g.M * g.N * sizeof(double));
+  l.cnt = carve(n_ids * sizeof(int));
+  l.qhi = carve(n_ids * sizeof(int));
+  l.qlo = carve(n_ids * sizeof(int));
+  l.ctl = carve(kExternalCtlBytes);
+  l.stats = carve(kExternalStatsBytes);
+  return l;
 }
 
 int make_geometry(long M, long N, int NB, int IB, Geometry* g, size_t smem_limit) {
@@ -274,12 +284,13 @@ static FactorTasks factor_tasks(const Geometry& g) {
   for (int i = 0; i < g.steps; i++) tiles += (long long)(g.NT - 1 - i) * (g.MT - i);
   FactorTasks f{update_columns(g, tiles, g.MT + g.steps, g.NB), fine_steps(g, false), 0};
   f.ids = coarse_task_ids(g, g.NB / f.cb) + (size_t)f.fine.ids;
-  if (external_bytes(g, coarse_task_ids(g, g.NC)) <= kNoAllocScratchBytes) {
-    if (f.fine.sub > 1 && external_bytes(g, f.ids) > kNoAllocScratchBytes) {
+  auto fits = [&](size_t ids) { return external_layout(g, ids).bytes <= kNoAllocScratchBytes; };
+  if (fits(coarse_task_ids(g, g.NC))) {
+    if (f.fine.sub > 1 && !fits(f.ids)) {
       f.fine = fine_steps(g, false, false, false);
       f.ids = coarse_task_ids(g, g.NB / f.cb) + (size_t)f.fine.ids;
     }
-    if (external_bytes(g, f.ids) > kNoAllocScratchBytes)
+    if (!fits(f.ids))
       f = FactorTasks{g.CB, FineSteps{}, coarse_task_ids(g, g.NC)};
   }
   return f;

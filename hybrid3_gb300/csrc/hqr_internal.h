@@ -160,10 +160,14 @@ constexpr int kExternalCtlBytes = 8 * 4;
 constexpr int kExternalStatsBytes = 14 * 8;
 // Number of task ids of the FP64 factorization DAG (size of cnt / qhi / qlo).
 size_t factor_task_ids(const Geometry& g);
-// The fixed scratch of hqr_geqrf_noalloc, and what it carves for n_ids task
-// ids: T factors, counters, two queues, control words, statistics.
+// The fixed scratch of hqr_geqrf_noalloc, and what it carves from it for n_ids
+// task ids (byte offsets, and the bytes in all): T factors, counters, two
+// queues, control words, statistics.
 constexpr size_t kNoAllocScratchBytes = size_t(64) << 20;
-size_t external_bytes(const Geometry& g, size_t n_ids);
+struct ExternalLayout {
+  size_t T, cnt, qhi, qlo, ctl, stats, bytes;
+};
+ExternalLayout external_layout(const Geometry& g, size_t n_ids);
 // Enqueue the factorization DAG on caller-supplied scratch.
 int launch_factor_external(const Geometry& g, const ExternalScratch& x, double* dA, double* dTAU,
                            long long timeout_ns, cudaStream_t stream);

@@ -40,8 +40,6 @@ static __device__ __align__(256) unsigned char g_noalloc_scratch[hqr::kNoAllocSc
 std::mutex g_noalloc_mu;
 void* g_noalloc_addr[kMaxDevices] = {};
 
-size_t round256(size_t b) { return (b + 255) & ~size_t(255); }
-
 // Device address of the scratch on the current device, looked up on the first
 // call made with that device current and cached.
 int noalloc_scratch(unsigned char** out) {
@@ -70,44 +68,32 @@ extern "C" int hqr_geqrf_noalloc(long M, long N, int NB, int IB, double* dA, dou
   int rc = hqr::make_geometry(M, N, NB, IB, &g);
   if (rc != HQR_OK) return rc;
 
-  // carve the scratch: T factors | counters | two queues | control | stats
-  const size_t n_ids = hqr::factor_task_ids(g);
-  const size_t b_t = round256((size_t)M * (size_t)N * sizeof(double));
-  const size_t b_ids = round256(n_ids * sizeof(int));
-  const size_t b_ctl = round256(hqr::kExternalCtlBytes);
-  const size_t b_stats = round256(hqr::kExternalStatsBytes);
-  const size_t need = hqr::external_bytes(g, n_ids);
-  if (need > hqr::kNoAllocScratchBytes) {
+  const hqr::ExternalLayout l = hqr::external_layout(g, hqr::factor_task_ids(g));
+  if (l.bytes > hqr::kNoAllocScratchBytes) {
     fprintf(stderr,
             "hqr_geqrf_noalloc: a %ld x %ld matrix with NB = %d needs %zu bytes of scratch; "
             "the fixed scratch holds %zu bytes\n",
-            M, N, NB, need, hqr::kNoAllocScratchBytes);
+            M, N, NB, l.bytes, hqr::kNoAllocScratchBytes);
     return HQR_ERR_UNSUPPORTED;
   }
   unsigned char* base = nullptr;
   rc = noalloc_scratch(&base);
   if (rc != HQR_OK) return rc;
   hqr::ExternalScratch x;
-  size_t off = 0;
-  x.T = reinterpret_cast<double*>(base + off);
-  off += b_t;
-  x.cnt = reinterpret_cast<int*>(base + off);
-  off += b_ids;
-  x.qhi = reinterpret_cast<int*>(base + off);
-  off += b_ids;
-  x.qlo = reinterpret_cast<int*>(base + off);
-  off += b_ids;
-  x.ctl = reinterpret_cast<unsigned*>(base + off);
-  off += b_ctl;
-  x.stats = reinterpret_cast<unsigned long long*>(base + off);
+  x.T = reinterpret_cast<double*>(base + l.T);
+  x.cnt = reinterpret_cast<int*>(base + l.cnt);
+  x.qhi = reinterpret_cast<int*>(base + l.qhi);
+  x.qlo = reinterpret_cast<int*>(base + l.qlo);
+  x.ctl = reinterpret_cast<unsigned*>(base + l.ctl);
+  x.stats = reinterpret_cast<unsigned long long*>(base + l.stats);
 
   cudaStream_t s = (cudaStream_t)stream;
   // The array keeps the previous call's contents.  The control words and the
   // statistics must start at zero; the counters and queues are written by the
   // DAG's init kernel, and every T block is written by its panel task before
   // any update reads it.
-  cudaError_t e = cudaMemsetAsync(x.ctl, 0, b_ctl, s);
-  if (e == cudaSuccess) e = cudaMemsetAsync(x.stats, 0, b_stats, s);
+  cudaError_t e = cudaMemsetAsync(x.ctl, 0, hqr::kExternalCtlBytes, s);
+  if (e == cudaSuccess) e = cudaMemsetAsync(x.stats, 0, hqr::kExternalStatsBytes, s);
   if (e != cudaSuccess) return hqr::record_cuda_error(e, "hqr_geqrf_noalloc: scratch reset");
   rc = hqr::launch_factor_external(g, x, dA, dTAU, 20000LL * 1000000LL, s);
   if (rc != HQR_OK) return rc;
