@@ -56,13 +56,13 @@ int make_geometry(long M, long N, int NB, int IB, Geometry* g, size_t smem_limit
   cb -= cb % 8;
   for (; cb >= 8; cb -= 8) {
     if (NB % cb != 0) continue;
-    TileShape sh{NB, w, cb, NB >= 512 ? 64 : kRC};
+    TileShape sh{NB, w, cb, NB >= 512 ? 64 : kRC, cb};
     if ((size_t)SmemPlan::make(sh).total * sizeof(double) <= smem_cap) break;
   }
   if (cb < 8) return HQR_ERR_UNSUPPORTED;
   g->CB = cb;
   g->NC = NB / cb;
-  TileShape sh{NB, w, cb, NB >= 512 ? 64 : kRC};
+  TileShape sh{NB, w, cb, NB >= 512 ? 64 : kRC, cb};
   SmemPlan sp = SmemPlan::make(sh);
   g->smem_bytes = (size_t)sp.total * sizeof(double);
   if (g->smem_bytes > smem_cap) return HQR_ERR_UNSUPPORTED;
@@ -73,7 +73,7 @@ int make_geometry(long M, long N, int NB, int IB, Geometry* g, size_t smem_limit
 }
 
 static TileShape shape_of(const Geometry& g) {
-  return TileShape{g.NB, g.w, g.CB, g.NB >= 512 ? 64 : kRC};
+  return TileShape{g.NB, g.w, g.CB, g.NB >= 512 ? 64 : kRC, g.CB};
 }
 
 int dag_workspace_reserve(DagWorkspace* ws, size_t n_ids) {
@@ -259,7 +259,8 @@ static int update_columns(const Geometry& g, long long tiles, long long path, in
 static void set_columns(DagParams& p, const Geometry& g, int cb, int cols) {
   p.sh = shape_of(g);
   if (p.oz) return;
-  p.ucols = cb;
+  p.sh.CB = cb;
+  if (p.mode != kModeFactor) p.sh.PB = cb;
   p.NC = (cols + cb - 1) / cb;
   p.count_every = g.CB / cb;
 }
@@ -557,7 +558,7 @@ static DagParams batch_matrix_params(bool apply, const Geometry& g, int nrhs) {
       int cb = (nrhs + 7) / 8 * 8;
       while (cb < g.CB && g.NB % cb != 0) cb += 8;
       if (cb > g.CB) cb = g.CB;
-      p.sh.CB = cb;
+      p.sh.CB = p.sh.PB = cb;
       p.NC = (nrhs + cb - 1) / cb;
     }
   }

@@ -87,13 +87,9 @@ struct DagParams {
   int mode;
   int MT, NT, CT, NC, steps, J;   // J = tile columns spanned by update ids
   int nblk;                        // panel inner blocks per panel task id (factorization: NB / w)
-  // FP64, one matrix: columns of an update task, at most sh.CB, the tile's
-  // nominal column block.  A panel block's own trailing update keeps the nominal
-  // strips (300 x 4 tiles of order 256, whole panel blocks in the first step:
-  // factorization 414 ms, 517 with the update tasks' 8 columns).  Of tasks
-  // narrower than the nominal block one in count_every is counted in the
-  // statistics (0, 1: all).
-  int ucols, count_every;
+  // update tasks that are narrower than the tile's nominal column block: one
+  // in count_every is counted in the statistics (0, 1: all)
+  int count_every;
   // Domain tree (tree > 0): at step i the tile rows i.. are cut into domains of
   // `tree` tiles; each domain runs the flat TS chain on its own top tile, then
   // the domain tops' R are merged into R(i, i) one after the other by TT
@@ -741,7 +737,7 @@ __global__ void __launch_bounds__(kThreads, BATCH ? 2 : 1) dag_exec_kernel(DagPa
     load_local(p, s_b, gid);
     const DagParams& q = local_params(p, s_b);
     const int id = gid - q.id_base;
-    const int NB = q.sh.NB, ub = BATCH ? q.sh.CB : q.ucols;
+    const int NB = q.sh.NB;
     const size_t tsz = (size_t)NB * NB;
     const TaskDesc t = decode(q, id);
     const long long c0 = clock64();
@@ -826,8 +822,8 @@ __global__ void __launch_bounds__(kThreads, BATCH ? 2 : 1) dag_exec_kernel(DagPa
           oz_exps = q.sexp + slot * oz::kSlots * NB;
           oz_bot = q.C + oc + (size_t)t.c * q.oz_cpt * oz::kN * NB;
           oz_col0 = (long long)t.j * NB + (long long)t.c * q.oz_cpt * oz::kN;
-        } else if (q.c_cols <= 0 || (long long)t.j * NB + (long long)t.c * ub < q.c_cols) {
-          task_larfb(q.A + ov, q.T + ov, q.C + oc, t.c * ub, ub, q.sh, smem, q.sp,
+        } else if (q.c_cols <= 0 || (long long)t.j * NB + (long long)t.c * q.sh.CB < q.c_cols) {
+          task_larfb(q.A + ov, q.T + ov, q.C + oc, t.c * q.sh.CB, q.sh.CB, q.sh, smem, q.sp,
                      applies_h(q.mode));
         }
         break;
@@ -846,9 +842,9 @@ __global__ void __launch_bounds__(kThreads, BATCH ? 2 : 1) dag_exec_kernel(DagPa
           oz_top = q.C + o1 + cofs;
           oz_bot = q.C + o2 + cofs;
           oz_col0 = (long long)t.j * NB + (long long)t.c * q.oz_cpt * oz::kN;
-        } else if (q.c_cols <= 0 || (long long)t.j * NB + (long long)t.c * ub < q.c_cols) {
-          task_ssrfb(q.C + o1, q.C + o2, q.A + ov, tt ? q.T2 + slot * tsz : q.T + ov, t.c * ub, ub, q.sh,
-                     smem, q.sp, applies_h(q.mode), tt);
+        } else if (q.c_cols <= 0 || (long long)t.j * NB + (long long)t.c * q.sh.CB < q.c_cols) {
+          task_ssrfb(q.C + o1, q.C + o2, q.A + ov, tt ? q.T2 + slot * tsz : q.T + ov, t.c * q.sh.CB,
+                     q.sh.CB, q.sh, smem, q.sp, applies_h(q.mode), tt);
         }
         break;
       }

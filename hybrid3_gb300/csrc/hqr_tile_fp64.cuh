@@ -35,6 +35,11 @@ struct TileShape {
   int w;    // inner block width = min(IB, kMaxW)
   int CB;   // columns per LARFB/SSRFB column-block task
   int RC;   // V row chunk
+  // columns of a strip of a panel block's own trailing update: the tile's
+  // nominal column block, also where the update tasks are narrower (300 x 4
+  // tiles of order 256, whole panel blocks in the first step: factorization 414
+  // ms, 517 with the update tasks' 8 columns)
+  int PB;
 };
 
 // Shared-memory carve-up, in doubles.  Computed identically on host and device.
@@ -43,13 +48,13 @@ struct SmemPlan {
   int total;
   __host__ __device__ static SmemPlan make(const TileShape& s) {
     SmemPlan p;
-    const int NB = s.NB, w = s.w, CB = s.CB;
+    const int NB = s.NB, w = s.w, CB = s.CB, PB = s.PB;
     // One region serves, one at a time: the GEQRT/TSQRT panel (NB x w), the
     // LARFB column block (NB x CB), the SSRFB pair A1|A2 (2 x NB x CB) and the
-    // TSQRT trailing chunk R-rows|A2 (w x CB + NB x CB).
+    // TSQRT trailing strip R-rows|A2 (w x PB + NB x PB).
     int region = NB * w;
     if (2 * NB * CB > region) region = 2 * NB * CB;
-    if (w * CB + NB * CB > region) region = w * CB + NB * CB;
+    if (w * PB + NB * PB > region) region = w * PB + NB * PB;
     int o = 0;
     p.off_c1 = o;
     p.off_c2 = o + NB * CB;                // SSRFB A2
@@ -58,8 +63,8 @@ struct SmemPlan {
     p.off_vt = o; o += w * w;              // unit-lower top of V / TSQRT R block
     p.off_t = o; o += w * w;               // T block
     p.off_g = o; o += w * w;               // Gram scratch of the T-block build
-    p.off_w = o; o += w * CB;
-    p.off_w2 = o; o += w * CB;
+    p.off_w = o; o += w * (CB > PB ? CB : PB);
+    p.off_w2 = o; o += w * (CB > PB ? CB : PB);
     p.off_part = o; o += 8 * kSplitItems;  // split-K partials (<= kSplitItems items x 8)
     p.off_red = o; o += kRedSlots;         // block reductions (kWarps) + broadcasts (4)
     p.off_tau = o; o += kMaxW;
@@ -952,8 +957,8 @@ __device__ void task_geqrt_blk(double* A, double* T, double* tau_g, const TileSh
     store_block(T + i0 + (size_t)i0 * NB, NB, sTb, w, w, w);
     for (int e = threadIdx.x; e < w; e += kThreads) stg_cg(tau_g + i0 + e, double(sTau[e]));
     __syncthreads();
-    for (int c0 = trailing ? i0 + w : NB; c0 < NB; c0 += sh.CB) {
-      const int ncol = min(sh.CB, NB - c0);
+    for (int c0 = trailing ? i0 + w : NB; c0 < NB; c0 += sh.PB) {
+      const int ncol = min(sh.PB, NB - c0);
       RT* sC = sm + sp.off_c1;
       __syncthreads();
       load_block(sC, NB, A + i0 + (size_t)c0 * NB, NB, m, ncol);
@@ -1045,10 +1050,10 @@ __device__ void task_tsqrt_blk(double* A1, double* A2, double* T, double* tau_g,
     store_block(T + i0 + (size_t)i0 * NB, NB, sTb, w, w, w);
     for (int e = threadIdx.x; e < w; e += kThreads) stg_cg(tau_g + i0 + e, double(sTau[e]));
     __syncthreads();
-    for (int c0 = trailing ? i0 + w : NB; c0 < NB; c0 += sh.CB) {
-      const int ncol = min(sh.CB, NB - c0);
+    for (int c0 = trailing ? i0 + w : NB; c0 < NB; c0 += sh.PB) {
+      const int ncol = min(sh.PB, NB - c0);
       RT* sCt = sm + sp.off_c1;  // w x ncol rows of R (the panel area is free now)
-      RT* sCb = sm + sp.off_c1 + w * sh.CB;  // NB x ncol of A2 after the R rows
+      RT* sCb = sm + sp.off_c1 + w * sh.PB;  // NB x ncol of A2 after the R rows
       __syncthreads();
       // A TT merge's block reflectors reach rows < i0 + w of A2 only: the rows
       // below belong to the domain top's own later blocks, which its chain may
@@ -1077,10 +1082,10 @@ __device__ void task_trailing(double* A1, double* A2, const double* T, const Til
   const int i0 = b * w;
   const int m = A2 ? NB : NB - i0;
   const double* V = A2 ? A2 + (size_t)i0 * NB : A1 + i0 + (size_t)i0 * NB;
-  for (int c0 = cbeg; c0 < cbeg + cols; c0 += sh.CB) {
-    const int ncol = min(sh.CB, cbeg + cols - c0);
+  for (int c0 = cbeg; c0 < cbeg + cols; c0 += sh.PB) {
+    const int ncol = min(sh.PB, cbeg + cols - c0);
     RT* sCt = sm + sp.off_c1;                                // the w x ncol rows of R (GEQRT: with the rows below)
-    RT* sCb = A2 ? sCt + w * sh.CB : sCt + w;
+    RT* sCb = A2 ? sCt + w * sh.PB : sCt + w;
     const int ldt = A2 ? w : NB;
     double* top = A1 + i0 + (size_t)c0 * NB;
     __syncthreads();
