@@ -238,18 +238,34 @@ static FineSteps fine_steps(const Geometry& g, bool split, bool fp32 = false, bo
 // Columns per FP64 update task: the tile's nominal block (g.CB), or fewer
 // where the longest chain of updates (`path` tasks) sets the pace rather than
 // all `tiles` of them (`cols` columns of data each) on every SM.  A task of cb
-// columns takes cb + c0 column times, c0 about 4, 14 at tile order 64
-// (measured, us, CB 64 / 32 / 16 / 8: NB 64 183 / 100 / 63 / 49; NB 128 635 /
-// 337 / 180 / 108; NB 256 - / 1251 / 674 / 414).
-static int update_columns(const Geometry& g, long long tiles, long long path, int cols) {
-  const double c0 = std::max(4.0, 57344.0 / ((double)g.NB * g.NB));
+// columns takes cb + c0 column times: c0 is 12 us and 6 us an inner block, in
+// columns of NB^2 / 1700 us each, and at least 4; 20 for tiles of order 512,
+// whose V goes through shared memory in chunks of 64 rows (us a link of Q^T C's
+// chain, CB 64 / 32 / 16 / 8: NB 32, w 8 - / 40.9 / 35.5 / 35.8, w 32 - / 40.2 /
+// 29.7 / 23.9; NB 64, w 16 175 / 98 / 64 / 51; NB 128 - / 310 / 169 / 103; NB 512
+// - / - / 1241 / 969).
+//
+// Q generation and the applications (`apply`) start with few tiles or end with
+// few, so that chain and work overlap in part only: three tenths of the smaller
+// count too, a gain has to be 8 %, and tiles of order 512 stay at their nominal
+// 16 columns unless the work stays below nine tenths of the chain.  A
+// factorization's chain has its panel blocks besides, and its tasks are
+// narrowed as if chain and work overlapped.  (ms, nominal / the narrower block
+// that the plain maximum takes: Q, 4 x 4 tiles of order 512 20.0 / 26.6; 20 x 20
+// of 32 1.69 / 1.89; 14 x 14 of 32 1.18 / 1.33, 1.04 with 16 columns.)  Tiles of
+// order 16 have nothing to cut (factorization of 20 x 20: 1.89 ms, 2.06 cut).
+static int update_columns(const Geometry& g, long long tiles, long long path, int cols, bool apply) {
+  const double c0 =
+      g.NB >= 512 ? 20.0 : std::max(4.0, 1700.0 * (12.0 + 6.0 * (g.NB / g.w)) / ((double)g.NB * g.NB));
   int best = g.CB;
   double t_best = 0.0;
-  for (int cb = g.CB; cb >= 8; cb -= 8) {
+  for (int cb = g.CB; cb >= (g.NB < 32 ? g.CB : 8); cb -= 8) {
     const long long tasks = tiles * ((cols + cb - 1) / cb);
     if (g.CB % cb != 0 || tasks > 0x0fffffffLL) continue;
-    const double t = (cb + c0) * std::max((double)path, (double)tasks / dag_sm_count());
-    if (cb == g.CB || t < 0.95 * t_best) {
+    const double chain = (double)path, work = (double)tasks / dag_sm_count();
+    if (apply && g.NB >= 512 && cb < g.CB && work > 0.9 * chain) continue;
+    const double t = (cb + c0) * (std::max(chain, work) + (apply ? 0.3 : 0.0) * std::min(chain, work));
+    if (cb == g.CB || t < (apply ? 0.92 : 0.95) * t_best) {
       best = cb;
       t_best = t;
     }
@@ -269,7 +285,7 @@ static void set_columns(DagParams& p, const Geometry& g, int cb, int cols) {
 static void set_apply_columns(DagParams& p, const Geometry& g, long long tiles, long long path, int CT,
                               long long ccols) {
   const int cols = CT == 1 && ccols > 0 && ccols < g.NB ? (int)ccols : g.NB;
-  set_columns(p, g, update_columns(g, tiles, path, cols), cols);
+  set_columns(p, g, update_columns(g, tiles, path, cols, true), cols);
 }
 
 // The FP64 factorization's update columns and fine steps.  The allocation-free
@@ -283,7 +299,7 @@ struct FactorTasks {
 static FactorTasks factor_tasks(const Geometry& g) {
   long long tiles = 0;
   for (int i = 0; i < g.steps; i++) tiles += (long long)(g.NT - 1 - i) * (g.MT - i);
-  FactorTasks f{update_columns(g, tiles, g.MT + g.steps, g.NB), fine_steps(g, false), 0};
+  FactorTasks f{update_columns(g, tiles, g.MT + g.steps, g.NB, false), fine_steps(g, false), 0};
   f.ids = coarse_task_ids(g, g.NB / f.cb) + (size_t)f.fine.ids;
   auto fits = [&](size_t ids) { return external_layout(g, ids).bytes <= kNoAllocScratchBytes; };
   if (fits(coarse_task_ids(g, g.NC))) {
@@ -336,7 +352,7 @@ static long long plan_apply_ids(const DagParams& f, const Geometry& g, int chain
   }
   const long long path = chain + g.steps;
   auto ids = [&](long long tiles, int CT) {
-    long long nc = f.oz ? g.NB / oz::kN / oz_chunks(tiles, path) : g.NB / update_columns(g, tiles, path, g.NB);
+    long long nc = f.oz ? g.NB / oz::kN / oz_chunks(tiles, path) : g.NB / update_columns(g, tiles, path, g.NB, true);
     if (!f.oz && CT == 1) nc = g.NB / 8;   // (few right-hand sides in one tile column: any width)
     return g.steps * ((long long)g.MT + f.dmax + ((long long)g.MT + f.dmax) * CT * nc);
   };
@@ -490,7 +506,7 @@ int launch_build_q(const Geometry& g, DagWorkspace* ws, const double* dA, double
   long long tiles = 0;
   for (int i = 0; i < g.steps; i++) tiles += (long long)(g.NT - i) * (g.MT - i);
   set_oz(p, g, ozw, oz_chunks(tiles, g.MT + g.steps));
-  set_columns(p, g, update_columns(g, tiles, g.MT + g.steps, g.NB), g.NB);
+  set_columns(p, g, update_columns(g, tiles, g.MT + g.steps, g.NB, true), g.NB);
   p.prep = 0;
   p.nblk = 1;
   p.skip_panels = rebuild_t ? 0 : 1;   // as in launch_apply_qt (split: T from its own slot)
