@@ -196,11 +196,7 @@ static int run_dag(DagParams& p, DagWorkspace* ws, const Geometry& g, cudaStream
 // the shorter chain gains.  Measured, against whole panel blocks: FP64 n =
 // 2048, NB 256: factorization 73 -> 38 ms; n = 4096: 155 -> 118 ms; split n =
 // 3072 (against blocks that released their dependents in phases): QR + Q 35.7
-// -> 28.4 ms; split n = 16384 unchanged.  With FP32 panels only the last step is
-// one (no tiles left): their blocks take half the time and are latency, not work
-// (factorization, ms, none / the last step: 4 x 4 tiles 3.46 / 3.39, 16 x 16
-// 14.7 / 14.6, 256 x 64 292 / 295, 1000 x 2 103.1 / 104.5; 32768 x 8192 then:
-// 355 / - , 356 from 300 tiles on, 382 from 6000).
+// -> 28.4 ms; split n = 16384 unchanged.  FP32 panels: fine_tiles_fp32.
 //
 // Such a task takes a part of a block's w columns: the chain through a tile is
 // its panel blocks and the first part after each, and a part of 8 / 16 / 32
@@ -212,14 +208,35 @@ static int run_dag(DagParams& p, DagWorkspace* ws, const Geometry& g, cudaStream
 // n = 3072: 21.4 / - / 22.2; but 594 panel tiles: FP64 38400 x 1024, NB 256:
 // 118 / 112.2 / 111.8, split 19200 x 512: 18.2 / - / 14.6), and FP64 parts of
 // 16 beyond that.
+//
+// FP32 panel blocks take half the time and are latency, not work, and the
+// scheduler hands out about two of the small tasks a microsecond.  They are cut
+// by what the whole factorization is: `load` is its work on every SM (an update
+// 50 us, a panel tile 1 ms) over its chain (a tile down a column 105 us, a step
+// 660 us).  Small loads: in every step; matrices that are not tall gain somewhat
+// longer, and up to a load of 1 in their last steps (300 tiles left); none
+// beyond.  Factorization, ms, none / from 300 tiles on / all steps, in tiles:
+//   load to 0.45: 4 x 4 3.49 / 2.91 / 2.92, 30 x 6 7.88 / 6.01 / 5.98, 100 x 3
+//     12.5 / 7.5 / 7.5, 256 x 4 29.5 / 29.7 / 19.5, 1000 x 2 103 / 105 / 54, 64 x 8
+//     13.2 / 13.0 / 11.1, 40 x 40 39.3 / 37.3 / 36.0, 12 x 80 11.7 / 11.1 / 9.8
+//   0.52 .. 1: 32 x 64 31.9 / 31.1 / 28.3, 48 x 48 47.7 / 45.7 / 47.6, 64 x 64 73.7
+//     / 72.4 / 82.8; tall 400 x 8 48.5 / 48.8 / 56.5, 128 x 16 28.5 / 29.0 / 36.9
+//   above 1: 256 x 32 106 / 109 / 155, 256 x 64 293 / 296 / 396
 struct FineSteps {
   int from = 0, sub = 1;
   long long ids = 0, tasks = 0;
 };
-constexpr long long kFineTilesSplit = 6000, kFineTilesFp64 = 600, kFineTilesFp32 = 0;
+constexpr long long kFineTilesSplit = 6000, kFineTilesFp64 = 600;
+static long long fine_tiles_fp32(const Geometry& g) {   // -1: no such steps
+  double work = 0.0;
+  for (int i = 0; i < g.steps; i++) work += (g.MT - i) * (1000.0 + 50.0 * (g.NT - 1 - i));
+  const double load = work / (dag_sm_count() * (105.0 * g.MT + 660.0 * g.steps));
+  const bool tall = g.MT > 3 * g.steps;
+  return load <= (tall ? 0.45 : 0.53) ? 0x7fffffffLL : load <= 1.0 && !tall ? 300 : -1;
+}
 static FineSteps fine_steps(const Geometry& g, bool split, bool fp32 = false, bool parts = true) {
   FineSteps f;
-  const long long nblk = g.NB / g.w, tiles = fp32 ? kFineTilesFp32 : split ? kFineTilesSplit : kFineTilesFp64;
+  const long long nblk = g.NB / g.w, tiles = fp32 ? fine_tiles_fp32(g) : split ? kFineTilesSplit : kFineTilesFp64;
   while (f.from < g.steps && (long long)(g.NT - f.from - 1) * (g.MT - f.from - 1) > tiles) f.from++;
   if (nblk < 2) return f;
   long long panels = 0;
