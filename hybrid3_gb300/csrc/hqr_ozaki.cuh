@@ -20,21 +20,20 @@
 //     accumulated in one FP32 TMEM accumulator, < 7 * 2^21 < 2^24 (the two
 //     products with the top digit are at most 2^13);
 //   * the 8 t-group accumulators (8 x 64 TMEM columns = the whole TMEM) are
-//     recombined exactly in 64-bit integers (two Horner chains in base 2^8,
-//     V = hi 2^32 + lo, up to 77 bits), shifted right only as far as V's bit
-//     length requires to fit 63 bits, rounding to odd, and converted to FP64
-//     with integer operations: the result is V correctly rounded, once.  The
+//     recombined exactly (two 64-bit Horner chains in base 2^8, V = hi 2^32 +
+//     lo, up to 77 bits, as three 32-bit words), normalised, rounded once to
+//     the nearest FP64 value and encoded with 32-bit integer operations.  The
 //     dropped products weigh < 2^-58 of rowmax(X) * colmax(Y) * K.
 //
 // The left operands are sliced once per panel tile into HBM, already in the
 // tcgen05 K-major core-matrix layout, so each 16-deep K chunk of all 8 slices
-// arrives with one 32 KiB bulk TMA copy.  The right operand lives in shared
-// memory (staged from HBM for the first product of an update, written there
-// by the previous product's epilogue otherwise) and is sliced chunk by chunk
-// into a double-buffered stage while the MMAs of the previous chunk run.
-// MMAs are issued by one thread (M = 128, N = 64, K = 16, FP16 x FP16 ->
-// FP32).  Every mbarrier wait is bounded; on time-out the error word is set
-// and the task is abandoned.
+// arrives with one 32 KiB bulk TMA copy (a ring of kAStages).  The right operand
+// lives in shared memory (staged from HBM for the first product of an update,
+// written there by the previous product's epilogue otherwise) and is sliced
+// chunk by chunk into a ring of kBStages, ahead of the MMAs.  MMAs are issued by
+// one elected lane of warp 0, the copies by one lane of warp 1 (M = 128, N = 64,
+// K = 16, FP16 x FP16 -> FP32).  Every mbarrier wait is bounded; on time-out the
+// error word is set and the task is abandoned.
 #pragma once
 #include <cstdint>
 #include "hqr_common.cuh"

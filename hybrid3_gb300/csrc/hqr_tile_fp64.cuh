@@ -421,7 +421,9 @@ __device__ __forceinline__ double f64_of(float f) {
 // 4); s = sqrt(f) by coupled Newton steps on sqrt and its inverse from an FP32
 // seed (Goldschmidt's iteration, residual taken with an FMA); 1 / (|a| 2^-h +
 // s) from an FP32 seed by one third-order (Householder) step.  Against the
-// exact values: tau 0.6, beta 0.8, scal 1.2 units in the last place at most.
+// exact values, restated on the host for 2 10^7 pairs a, ss with seeds up to
+// two units off: tau 1.5, beta 0.9, scal 2.8 units in the last place at most;
+// with square root and divisions 2.2, 0.9 and 2.8.
 __device__ __forceinline__ void larfg_newton(double a, double ss, double& tau, double& scal, double& beta) {
   const double n2 = fma(a, a, ss);
   const int hi = __double2hiint(n2), lo = __double2loint(n2);
