@@ -265,7 +265,9 @@ static FineSteps fine_steps(const Geometry& g, bool split, bool fp32 = false, bo
 // Q generation and the applications (`apply`) start with few tiles or end with
 // few, so that chain and work overlap in part only: three tenths of the smaller
 // count too, a gain has to be 8 %, and tiles of order 512 stay at their nominal
-// 16 columns unless the work stays below nine tenths of the chain.  A
+// 16 columns unless the work stays below nine tenths of the chain, which is one
+// task shorter than `path` (the last task of a step's column begins the next
+// step; Q^T C of one tile on 3 tile columns: 1.67 ms, 2.41 cut).  A
 // factorization's chain has its panel blocks besides, and its tasks are
 // narrowed as if chain and work overlapped.  (ms, nominal / the narrower block
 // that the plain maximum takes: Q, 4 x 4 tiles of order 512 20.0 / 26.6; 20 x 20
@@ -280,7 +282,7 @@ static int update_columns(const Geometry& g, long long tiles, long long path, in
     const long long tasks = tiles * ((cols + cb - 1) / cb);
     if (g.CB % cb != 0 || tasks > 0x0fffffffLL) continue;
     const double chain = (double)path, work = (double)tasks / dag_sm_count();
-    if (apply && g.NB >= 512 && cb < g.CB && work > 0.9 * chain) continue;
+    if (apply && g.NB >= 512 && cb < g.CB && work > 0.9 * (chain - 1.0)) continue;
     const double t = (cb + c0) * (std::max(chain, work) + (apply ? 0.3 : 0.0) * std::min(chain, work));
     if (cb == g.CB || t < (apply ? 0.92 : 0.95) * t_best) {
       best = cb;
