@@ -265,15 +265,17 @@ static FineSteps fine_steps(const Geometry& g, bool split, bool fp32 = false, bo
 // Q generation and the applications (`apply`) start with few tiles or end with
 // few, so that chain and work overlap in part only: three tenths of the smaller
 // count too, a gain has to be 8 %, and tiles of order 512 stay at their nominal
-// 16 columns unless the work stays below nine tenths of the chain, which is one
-// task shorter than `path` (the last task of a step's column begins the next
-// step; Q^T C of one tile on 3 tile columns: 1.67 ms, 2.41 cut).  A
-// factorization's chain has its panel blocks besides, and its tasks are
+// 16 columns unless the work stays below nine tenths of the chain and the tasks
+// of one of its links (a tile, on all CT tile columns of C) are one wave (ms,
+// nominal / 8 columns, MT x NT on CT: 192 tasks a link, 1 x 1 on 3 1.65 / 2.41,
+// 2 x 1 on 3 4.40 / 6.75; 128 a link, 3 x 2 on 2 9.91 / 8.96, 3 x 3 on 2 11.45 /
+// 10.13).  A factorization's chain has its panel blocks besides, and its tasks are
 // narrowed as if chain and work overlapped.  (ms, nominal / the narrower block
 // that the plain maximum takes: Q, 4 x 4 tiles of order 512 20.0 / 26.6; 20 x 20
 // of 32 1.69 / 1.89; 14 x 14 of 32 1.18 / 1.33, 1.04 with 16 columns.)  Tiles of
 // order 16 have nothing to cut (factorization of 20 x 20: 1.89 ms, 2.06 cut).
-static int update_columns(const Geometry& g, long long tiles, long long path, int cols, bool apply) {
+static int update_columns(const Geometry& g, long long tiles, long long path, int cols, int CT) {
+  const bool apply = CT > 0;   // (0: a factorization)
   const double c0 =
       g.NB >= 512 ? 20.0 : std::max(4.0, 1700.0 * (12.0 + 6.0 * (g.NB / g.w)) / ((double)g.NB * g.NB));
   int best = g.CB;
@@ -282,7 +284,8 @@ static int update_columns(const Geometry& g, long long tiles, long long path, in
     const long long tasks = tiles * ((cols + cb - 1) / cb);
     if (g.CB % cb != 0 || tasks > 0x0fffffffLL) continue;
     const double chain = (double)path, work = (double)tasks / dag_sm_count();
-    if (apply && g.NB >= 512 && cb < g.CB && work > 0.9 * (chain - 1.0)) continue;
+    const long long link = (long long)CT * ((cols + cb - 1) / cb);
+    if (apply && g.NB >= 512 && cb < g.CB && (work > 0.9 * chain || link > dag_sm_count())) continue;
     const double t = (cb + c0) * (std::max(chain, work) + (apply ? 0.3 : 0.0) * std::min(chain, work));
     if (cb == g.CB || t < (apply ? 0.92 : 0.95) * t_best) {
       best = cb;
@@ -304,7 +307,7 @@ static void set_columns(DagParams& p, const Geometry& g, int cb, int cols) {
 static void set_apply_columns(DagParams& p, const Geometry& g, long long tiles, long long path, int CT,
                               long long ccols) {
   const int cols = CT == 1 && ccols > 0 && ccols < g.NB ? (int)ccols : g.NB;
-  set_columns(p, g, update_columns(g, tiles, path, cols, true), cols);
+  set_columns(p, g, update_columns(g, tiles, path, cols, CT), cols);
 }
 
 // The FP64 factorization's update columns and fine steps.  The allocation-free
@@ -318,7 +321,7 @@ struct FactorTasks {
 static FactorTasks factor_tasks(const Geometry& g) {
   long long tiles = 0;
   for (int i = 0; i < g.steps; i++) tiles += (long long)(g.NT - 1 - i) * (g.MT - i);
-  FactorTasks f{update_columns(g, tiles, g.MT + g.steps, g.NB, false), fine_steps(g, false), 0};
+  FactorTasks f{update_columns(g, tiles, g.MT + g.steps, g.NB, 0), fine_steps(g, false), 0};
   f.ids = coarse_task_ids(g, g.NB / f.cb) + (size_t)f.fine.ids;
   auto fits = [&](size_t ids) { return external_layout(g, ids).bytes <= kNoAllocScratchBytes; };
   if (fits(coarse_task_ids(g, g.NC))) {
@@ -371,7 +374,7 @@ static long long plan_apply_ids(const DagParams& f, const Geometry& g, int chain
   }
   const long long path = chain + g.steps;
   auto ids = [&](long long tiles, int CT) {
-    long long nc = f.oz ? g.NB / oz::kN / oz_chunks(tiles, path) : g.NB / update_columns(g, tiles, path, g.NB, true);
+    long long nc = f.oz ? g.NB / oz::kN / oz_chunks(tiles, path) : g.NB / update_columns(g, tiles, path, g.NB, CT);
     if (!f.oz && CT == 1) nc = g.NB / 8;   // (few right-hand sides in one tile column: any width)
     return g.steps * ((long long)g.MT + f.dmax + ((long long)g.MT + f.dmax) * CT * nc);
   };
@@ -525,7 +528,7 @@ int launch_build_q(const Geometry& g, DagWorkspace* ws, const double* dA, double
   long long tiles = 0;
   for (int i = 0; i < g.steps; i++) tiles += (long long)(g.NT - i) * (g.MT - i);
   set_oz(p, g, ozw, oz_chunks(tiles, g.MT + g.steps));
-  set_columns(p, g, update_columns(g, tiles, g.MT + g.steps, g.NB, true), g.NB);
+  set_columns(p, g, update_columns(g, tiles, g.MT + g.steps, g.NB, g.NT), g.NB);
   p.prep = 0;
   p.nblk = 1;
   p.skip_panels = rebuild_t ? 0 : 1;   // as in launch_apply_qt (split: T from its own slot)
