@@ -658,9 +658,12 @@ __device__ __forceinline__ bool panel_qr(double* R, int ldr, double* A, int lda,
           double* aj = A + (size_t)(c + 1 + it) * lda;
           bool whole = moves;   // a -= f x with f as one factor
           if (Larfg::kSplitFactor) {
-            // (a factor that is not in range is two: a -= (t x) d)
+            // a factor that is not in range is two, a -= (t x) d, and so is one
+            // whose products can be exact (its low word is zero): the column is
+            // then a short multiple of x, 1 or 2 of it, say, and would become
+            // exactly zero instead of rounding errors (see the convention)
             const unsigned fh = (unsigned)__double2hiint(fq) & 0x7fffffffu;
-            whole = fh >= kHiExp(-960) && fh < kHiExp(960);
+            whole = fh >= kHiExp(-960) && fh < kHiExp(960) && __double2loint(fq) != 0;
             const double dq = __shfl_sync(0xffffffffu, d, q);
             for (int r = r0 + lane; r < m && !whole; r += 32) aj[r] = fma(-(t * x[r]), dq, aj[r]);
           }
